@@ -377,6 +377,12 @@ tg_status tg_gemm_host(int64_t M, int64_t N, int64_t K, const double* A, int64_t
                        const double* B, int64_t sBk, int64_t sBn, double* C, int64_t sCm, int64_t sCn,
                        int prec);
 
+/* The same for complex operands ((re, im) pairs; FP64 DMMA), each optionally
+ * conjugated. */
+tg_status tg_gemm_host_complex(int64_t M, int64_t N, int64_t K, const double* A, int64_t sAm, int64_t sAk,
+                               const double* B, int64_t sBk, int64_t sBn, double* C, int64_t sCm, int64_t sCn,
+                               int conj_a, int conj_b);
+
 /* Orthonormal basis of the span of a real column-major n x k host panel Y
  * (in place) by the engine's shifted CholeskyQR: `passes` passes, the first
  * two shifted, a perturbation of relative size 1e-14 after the first, all in

@@ -2423,35 +2423,45 @@ void gemm(const T* A, const T* B, T* C, const GemmDesc& d, cudaStream_t st) {
   // up to two CTAs per SM (the kernel's occupancy), K chunks of at least 128
   if (d.batch == 1 && tiles < 148 && d.K >= 256)
     split = std::min<int64_t>(std::max<int64_t>(1, 296 / tiles), (d.K + 127) / 128);
-  if (split <= 1) {
+  // all chunks in one launch (z = chunk, the last one possibly shorter), then an FP64 sum
+  const int64_t chunk = (d.K + split - 1) / split;
+  const int64_t chunk16 = split > 1 ? (chunk + GBK - 1) / GBK * GBK : d.K;  // multiple of the k tile
+  const int64_t nparts = (d.K + chunk16 - 1) / chunk16;
+  // small tiles where the large ones would leave most of the SMs idle
+  const double cycles = gemm_tile_cycles(d, GBM, nf > 0 ? 8 * nf : GBN, nparts, chunk16, CPLX);
+  // the second launch of a split product and its sums: about 2.5 us
+  const double sums = 5000.0;
+  if (nparts <= kTilePartsMax &&
+      gemm_tiles<T>(A, B, C, d, nparts, chunk16, cycles + (nparts > 1 ? sums : 0.0), nullptr, st))
+    return;
+  if (nparts <= 1) {
     launch(grid, GemmParams<T>{A, B, C, d});
     TG_CHECK_LAUNCH();
     count_launch();
     return;
   }
-  // all chunks in one launch (z = chunk, the last one possibly shorter), then an FP64 sum
-  const int64_t chunk = (d.K + split - 1) / split;
-  const int64_t chunk16 = (chunk + GBK - 1) / GBK * GBK;  // multiple of the k tile
-  const int64_t nparts = (d.K + chunk16 - 1) / chunk16;
   void* buf = nullptr;
   TG_CUDA(cudaMallocAsync(&buf, sizeof(T) * nparts * d.M * d.N, st));
   T* parts = static_cast<T*>(buf);
-  GemmDesc g = d;
-  g.sCm = d.N;
-  g.sCn = 1;
-  g.accumulate = false;
-  g.K = chunk16;
-  g.klast = d.K - (nparts - 1) * chunk16;
-  g.batch = nparts;
-  g.bA = chunk16 * d.sAk;
-  g.bB = chunk16 * d.sBk;
-  g.bC = d.M * d.N;
-  launch(dim3(grid.x, grid.y, static_cast<unsigned>(nparts)), GemmParams<T>{A, B, parts, g});
-  TG_CHECK_LAUNCH();
+  if (!gemm_tiles<T>(A, B, C, d, nparts, chunk16, cycles, parts, st)) {
+    GemmDesc g = d;
+    g.sCm = d.N;
+    g.sCn = 1;
+    g.accumulate = false;
+    g.K = chunk16;
+    g.klast = d.K - (nparts - 1) * chunk16;
+    g.batch = nparts;
+    g.bA = chunk16 * d.sAk;
+    g.bB = chunk16 * d.sBk;
+    g.bC = d.M * d.N;
+    launch(dim3(grid.x, grid.y, static_cast<unsigned>(nparts)), GemmParams<T>{A, B, parts, g});
+    TG_CHECK_LAUNCH();
+    count_launch();
+  }
   splitk_reduce_kernel<T><<<num_blocks(d.M * d.N, 256), 256, 0, st>>>(parts, static_cast<int>(nparts), d.M, d.N,
                                                                        C, d.sCm, d.sCn, d.accumulate);
   TG_CHECK_LAUNCH();
-  count_launch(2);
+  count_launch();
   TG_CUDA(cudaFreeAsync(buf, st));
 }
 

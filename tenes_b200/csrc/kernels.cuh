@@ -76,6 +76,17 @@ bool gemm_specialised(const GemmDesc& d);
 // other shape.  gemm() tries it first at both precisions (it is exact FP64).
 bool gemm_skinny(const double* A, const double* B, double* C, const GemmDesc& d, cudaStream_t st);
 
+// FP64 product on small CTA tiles (tile_gemm.cu), K in `nparts` parts of
+// `kchunk`, where its expected cycles are below `other_cycles`; else returns
+// false, launching nothing.  The parts are summed in the launch (nparts <=
+// kTilePartsMax), or written to `parts` where that is not null.
+// gemm_tile_cycles: the expected cycles on bm x bn tiles.
+constexpr int64_t kTilePartsMax = 8;
+template <typename T>
+bool gemm_tiles(const T* A, const T* B, T* C, const GemmDesc& d, int64_t nparts, int64_t kchunk, double other_cycles,
+                T* parts, cudaStream_t st);
+double gemm_tile_cycles(const GemmDesc& d, int64_t bm, int64_t bn, int64_t nparts, int64_t kchunk, bool complex_values);
+
 // True (and cleared) when a tcgen05 product gave up waiting for its tensor
 // cores since the last call.  Synchronises the device.
 bool tc_fault_take();

@@ -383,6 +383,12 @@ tg_status tg_gemm_host_complex(int64_t M, int64_t N, int64_t K, const double* A,
                                const double* B, int64_t sBk, int64_t sBn, double* C, int64_t sCm, int64_t sCn,
                                int conj_a, int conj_b);
 
+/* SVD A W = U S of one row-major n x n host matrix by the engine's one-sided
+ * Jacobi ((re, im) pairs when is_complex; n <= 119 real, 84 complex), singular
+ * values descending; circle != 0: the form the randomised projectors use.  For
+ * tests of the kernels; not part of the CTMRG path. */
+tg_status tg_jacobi_host(int64_t n, int is_complex, int circle, const double* A, double* U, double* S, double* W);
+
 /* Orthonormal basis of the span of a real column-major n x k host panel Y
  * (in place) by the engine's shifted CholeskyQR: `passes` passes, the first
  * two shifted, a perturbation of relative size 1e-14 after the first, all in

@@ -370,6 +370,38 @@ extern "C" tg_status tg_gemm_host_complex(int64_t M, int64_t N, int64_t K, const
   });
 }
 
+namespace {
+template <typename T>
+void jacobi_host(int64_t n, bool circle, const double* A, double* U, double* S, double* W) {
+  cudaStream_t st;
+  TG_CUDA(cudaStreamCreate(&st));
+  T* d = nullptr;  // A, U, W
+  double* s = nullptr;
+  TG_CUDA(cudaMalloc(&d, sizeof(T) * 3 * n * n));
+  TG_CUDA(cudaMalloc(&s, sizeof(double) * n));
+  TG_CUDA(cudaMemcpyAsync(d, A, sizeof(T) * n * n, cudaMemcpyHostToDevice, st));
+  tg::jacobi_svd<T>(d, n, d + n * n, s, d + 2 * n * n, circle, st);
+  TG_CUDA(cudaMemcpyAsync(U, d + n * n, sizeof(T) * n * n, cudaMemcpyDeviceToHost, st));
+  TG_CUDA(cudaMemcpyAsync(W, d + 2 * n * n, sizeof(T) * n * n, cudaMemcpyDeviceToHost, st));
+  TG_CUDA(cudaMemcpyAsync(S, s, sizeof(double) * n, cudaMemcpyDeviceToHost, st));
+  TG_CUDA(cudaStreamSynchronize(st));
+  cudaFree(d);
+  cudaFree(s);
+  cudaStreamDestroy(st);
+}
+}  // namespace
+
+extern "C" tg_status tg_jacobi_host(int64_t n, int is_complex, int circle, const double* A, double* U, double* S,
+                                    double* W) {
+  return guard([&] {
+    if (!A || !U || !S || !W) tg::fail(TG_E_INPUT, "bad jacobi arguments");
+    if (n < 1 || n > (is_complex ? tg::jacobi_svd_max_k<tg::cplx>() : tg::jacobi_svd_max_k<double>()))
+      tg::fail(TG_E_INPUT, "jacobi: n out of range");
+    if (is_complex) jacobi_host<tg::cplx>(n, circle != 0, A, U, S, W);
+    else jacobi_host<double>(n, circle != 0, A, U, S, W);
+  });
+}
+
 extern "C" tg_status tg_gemm_group_host(int n, const int64_t* mnk, const int* flags, int is_complex,
                                         const double* A, const double* B, double* C) {
   return guard([&] {

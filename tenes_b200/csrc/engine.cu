@@ -829,7 +829,7 @@ struct EngineT final : Engine {
     // (The previous sweep's right singular vectors are no warm start here: T
     // is expressed in the CholeskyQR basis of Z, which rotates within the
     // kept subspace from sweep to sweep, so a cold start needs fewer sweeps.)
-    jacobi_svd<T>(Tm.p, k, Ur.p, s.p, Wr.p, st);  // T Wr = Ur S
+    jacobi_svd<T>(Tm.p, k, Ur.p, s.p, Wr.p, true, st);  // T Wr = Ur S
     DT<T> U = mm_rm(cm(Q.p, nrow, k), rm(Ur.p, k, k));
     DT<T> V = mm_rm(cm(Qz.p, ncol, k), rm(Wr.p, k, k));
     const int w = static_cast<int>(std::min<int64_t>(k, P.chi));
@@ -935,7 +935,7 @@ struct EngineT final : Engine {
         DT<T> Tm = mm_rm(ht(cm(Z.p, ncol, b)), cm(Qz.p, ncol, b));  // Q^H M Qz (b x b row-major)
         DT<T> Ur({b, b}, st), Wr({b, b}, st);
         DT<double> s({b}, st);
-        jacobi_svd<T>(Tm.p, b, Ur.p, s.p, Wr.p, st);  // T Wr = Ur S
+        jacobi_svd<T>(Tm.p, b, Ur.p, s.p, Wr.p, false, st);  // T Wr = Ur S
         DT<T> Y = mm_cm(m, cm(Qz.p, ncol, b));        // M Qz: nrow x b
         DT<T> MV1 = mm_cm(cm(Y.p, nrow, b), rm(Wr.p, b, b));  // M v_i
         DT<T> U1 = mm_cm(cm(Q.p, nrow, b), rm(Ur.p, b, b));   // u_i
@@ -1015,7 +1015,7 @@ struct EngineT final : Engine {
       DT<T> Q = transpose<T>(M, {0, 1}, st, true);  // column-major view: M^H
       orth_cm(Q, ncol, k);
       DT<T> B = mm_rm(rm(M.p, nrow, ncol), cm(Q.p, ncol, k));
-      jacobi_svd<T>(B.p, k, Ub.p, s.p, Wb.p, st);  // B Wb = Ub S
+      jacobi_svd<T>(B.p, k, Ub.p, s.p, Wb.p, true, st);  // B Wb = Ub S
       U = Ub;
       VT = transpose<T>(mm_rm(cm(Q.p, ncol, k), rm(Wb.p, k, k)), {1, 0}, st, true);
     } else {
@@ -1023,7 +1023,7 @@ struct EngineT final : Engine {
       DT<T> Q = transpose<T>(M, {1, 0}, st);  // column-major view: M
       orth_cm(Q, nrow, k);
       DT<T> B = mm_rm(ht(cm(Q.p, nrow, k)), rm(M.p, nrow, ncol));
-      jacobi_svd<T>(B.p, k, Ub.p, s.p, Wb.p, st);
+      jacobi_svd<T>(B.p, k, Ub.p, s.p, Wb.p, true, st);
       U = mm_rm(cm(Q.p, nrow, k), rm(Ub.p, k, k));
       VT = transpose<T>(Wb, {1, 0}, st, true);
     }
@@ -1741,7 +1741,7 @@ struct EngineT final : Engine {
       for (int k = 0; k < 4; ++k) h_ptrs[4 * i + k] = C[k][i].p;
     TG_CUDA(cudaMemcpyAsync(d_ptrs, h_ptrs, sizeof(T*) * cnt, cudaMemcpyHostToDevice, st));
     DT<double> out({cnt, static_cast<int64_t>(P.chi)}, st);
-    batched_spectrum<T>(d_ptrs, cnt, P.chi, out.p, nullptr, st);
+    batched_spectrum<T>(d_ptrs, cnt, P.chi, out.p, st);
     return out;
   }
 

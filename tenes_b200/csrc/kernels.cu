@@ -1,6 +1,6 @@
 // Hand-written sm_100a kernels of the CTMRG path: FP64 tensor-core (DMMA)
 // strided batched matrix product, leg permutation, max-abs normalisation,
-// projector truncation helpers and a batched one-sided Jacobi spectrum.
+// projector truncation helpers.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include <cuda_runtime.h>
@@ -1518,152 +1518,6 @@ __global__ void identity_kernel(T* __restrict__ out, int64_t e) {
   }
 }
 
-// ---------------------------------------------------------------------------
-// One-sided (Hestenes) Jacobi singular values, one CTA per n x n matrix.
-// Columns live in shared memory (column-major); each warp orthogonalises
-// disjoint column pairs of a round-robin schedule.  Converged when no pair of
-// a sweep needed a rotation (|a_p^H a_q| <= n u sqrt(|a_p|^2 |a_q|^2)), or
-// after 60 sweeps (the count is reported back).
-// ---------------------------------------------------------------------------
-// sum of |x|^2 over a shared-memory array (re [, im] planes), whole CTA
-template <bool CPLX>
-__device__ double block_sumsq(const double* re, const double* im, int len) {
-  __shared__ double wsum[32];
-  __shared__ double total;
-  double a = 0.0;
-  for (int i = threadIdx.x; i < len; i += blockDim.x) {
-    a += re[i] * re[i];
-    if constexpr (CPLX) a += im[i] * im[i];
-  }
-  for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-  if ((threadIdx.x & 31) == 0) wsum[threadIdx.x >> 5] = a;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    double b = (threadIdx.x < (blockDim.x >> 5)) ? wsum[threadIdx.x] : 0.0;
-    for (int o = 16; o > 0; o >>= 1) b += __shfl_xor_sync(0xffffffffu, b, o);
-    if (threadIdx.x == 0) total = b;
-  }
-  __syncthreads();
-  return total;
-}
-
-template <typename T, bool CPLX>
-__global__ void __launch_bounds__(256) jacobi_spectrum_kernel(const T* const* mats, int n,
-                                                                double* out, int* sweeps_used) {
-  extern __shared__ double sm[];
-  double* re = sm;                      // n*n column-major
-  double* im = sm + (CPLX ? n * n : 0);  // n*n (complex only)
-  double* nrm = sm + (CPLX ? 2 : 1) * n * n;  // n
-  __shared__ int rotated;
-  const T* M = mats[blockIdx.x];
-  for (int idx = threadIdx.x; idx < n * n; idx += blockDim.x) {
-    const int r = idx / n, c = idx % n;  // row-major source
-    const T v = M[idx];
-    re[c * n + r] = re_of(v);
-    if constexpr (CPLX) im[c * n + r] = im_of(v);
-  }
-  __syncthreads();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const int np = n + (n & 1);
-  const double tol = static_cast<double>(n) * 2.220446049250313e-16;
-  const double small2 = tol * tol * block_sumsq<CPLX>(re, im, n * n);  // rounding-noise columns
-  int sweep = 0;
-  for (; sweep < 60; ++sweep) {
-    if (threadIdx.x == 0) rotated = 0;
-    __syncthreads();
-    for (int rnd = 0; rnd < np - 1; ++rnd) {
-      for (int pr = warp; pr < np / 2; pr += nw) {
-        auto player = [&](int k) { return k == 0 ? 0 : ((k - 1 + rnd) % (np - 1)) + 1; };
-        int p = player(pr), q = player(np - 1 - pr);
-        if (p >= n || q >= n) continue;
-        if (p > q) {
-          int t = p;
-          p = q;
-          q = t;
-        }
-        double al = 0, be = 0, gr = 0, gi = 0;
-        for (int r = lane; r < n; r += 32) {
-          const double pr_ = re[p * n + r], qr_ = re[q * n + r];
-          al += pr_ * pr_;
-          be += qr_ * qr_;
-          gr += pr_ * qr_;
-          if constexpr (CPLX) {
-            const double pi_ = im[p * n + r], qi_ = im[q * n + r];
-            al += pi_ * pi_;
-            be += qi_ * qi_;
-            gr += pi_ * qi_;
-            gi += pr_ * qi_ - pi_ * qr_;  // Im(conj(a_p) a_q)
-          }
-        }
-        for (int o = 16; o > 0; o >>= 1) {
-          al += __shfl_xor_sync(0xffffffffu, al, o);
-          be += __shfl_xor_sync(0xffffffffu, be, o);
-          gr += __shfl_xor_sync(0xffffffffu, gr, o);
-          if constexpr (CPLX) gi += __shfl_xor_sync(0xffffffffu, gi, o);
-        }
-        const double g = CPLX ? hypot(gr, gi) : fabs(gr);
-        if (g == 0.0 || al <= small2 || be <= small2 || g <= tol * sqrt(al * be)) continue;
-        // phase e^{-i phi} with gamma = |gamma| e^{i phi}
-        const double ph_r = CPLX ? gr / g : (gr >= 0 ? 1.0 : -1.0);
-        const double ph_i = CPLX ? -gi / g : 0.0;
-        const double zeta = (be - al) / (2.0 * g);
-        const double t = (zeta >= 0 ? 1.0 : -1.0) / (fabs(zeta) + sqrt(1.0 + zeta * zeta));
-        const double c = 1.0 / sqrt(1.0 + t * t), s = c * t;
-        for (int r = lane; r < n; r += 32) {
-          const double apr = re[p * n + r];
-          const double api = CPLX ? im[p * n + r] : 0.0;
-          const double aqr = re[q * n + r];
-          const double aqi = CPLX ? im[q * n + r] : 0.0;
-          // b_q = a_q * e^{-i phi}
-          const double bqr = aqr * ph_r - aqi * ph_i;
-          const double bqi = aqr * ph_i + aqi * ph_r;
-          re[p * n + r] = c * apr - s * bqr;
-          re[q * n + r] = s * apr + c * bqr;
-          if constexpr (CPLX) {
-            im[p * n + r] = c * api - s * bqi;
-            im[q * n + r] = s * api + c * bqi;
-          }
-        }
-        if (lane == 0) rotated = 1;
-      }
-      __syncthreads();
-    }
-    __syncthreads();
-    const int any = rotated;
-    __syncthreads();
-    if (!any) break;
-  }
-  // column norms, normalised, sorted descending
-  for (int c = warp; c < n; c += nw) {
-    double a = 0;
-    for (int r = lane; r < n; r += 32) {
-      a += re[c * n + r] * re[c * n + r];
-      if constexpr (CPLX) a += im[c * n + r] * im[c * n + r];
-    }
-    for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-    if (lane == 0) nrm[c] = sqrt(a);
-  }
-  __syncthreads();
-  __shared__ double tot;
-  if (threadIdx.x < 32) {
-    double a = 0;
-    for (int c = lane; c < n; c += 32) a += nrm[c] * nrm[c];
-    for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-    if (lane == 0) tot = sqrt(a);
-  }
-  __syncthreads();
-  for (int c = threadIdx.x; c < n; c += blockDim.x) {
-    const double v = nrm[c];
-    int pos = 0;
-    for (int o = 0; o < n; ++o) {
-      const double w = nrm[o];
-      pos += (w > v) || (w == v && o < c);
-    }
-    out[static_cast<int64_t>(blockIdx.x) * n + pos] = tot > 0 ? v / tot : 0.0;
-  }
-  if (threadIdx.x == 0 && sweeps_used) sweeps_used[blockIdx.x] = sweep;
-}
-
 template <typename T>
 __global__ void counter_normal_kernel(T* __restrict__ out, int64_t rows, int64_t cols, uint64_t key_re,
                                       uint64_t key_im) {
@@ -1692,7 +1546,30 @@ __global__ void upper_to_rh_kernel(const T* __restrict__ acm, int64_t lda, int64
   }
 }
 
-// One-sided Jacobi SVD with vectors; see jacobi_svd() in kernels.cuh.
+// sum of |x|^2 over a shared-memory array (re [, im] planes), whole CTA
+template <bool CPLX>
+__device__ double block_sumsq(const double* re, const double* im, int len) {
+  __shared__ double wsum[32];
+  __shared__ double total;
+  double a = 0.0;
+  for (int i = threadIdx.x; i < len; i += blockDim.x) {
+    a += re[i] * re[i];
+    if constexpr (CPLX) a += im[i] * im[i];
+  }
+  for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+  if ((threadIdx.x & 31) == 0) wsum[threadIdx.x >> 5] = a;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    double b = (threadIdx.x < (blockDim.x >> 5)) ? wsum[threadIdx.x] : 0.0;
+    for (int o = 16; o > 0; o >>= 1) b += __shfl_xor_sync(0xffffffffu, b, o);
+    if (threadIdx.x == 0) total = b;
+  }
+  __syncthreads();
+  return total;
+}
+
+// One-sided Jacobi SVD with vectors, for the complex matrices of the randomised
+// projectors; see jacobi_svd_complex() in kernels.cuh.
 // Column pairs of a round-robin schedule are handled by groups of kJG lanes;
 // lane gl of a group holds rows gl + kJG i (i < RPL) of the pair's two
 // columns in registers for the round: one batch of loads, the dot product,
@@ -2936,23 +2813,6 @@ void identity(T* out, int64_t e, cudaStream_t st) {
   count_launch();
 }
 
-template <typename T>
-void batched_spectrum(const T* const* mats, int count, int n, double* out, int* sweeps_used,
-                      cudaStream_t st) {
-  if (count <= 0) return;
-  constexpr bool CPLX = is_cplx<T>::value;
-  // the matrix lives in shared memory: n <= 160 (real), 112 (complex)
-  const int nmax = CPLX ? 112 : 160;
-  if (n > nmax || n < 1)
-    fail(TG_E_INPUT, "batched_spectrum: 1 <= chi <= " + std::to_string(nmax) + " required");
-  const size_t smem = sizeof(double) * ((CPLX ? 2 : 1) * n * n + n);
-  ensure_dynamic_smem(reinterpret_cast<const void*>(jacobi_spectrum_kernel<T, CPLX>), smem);
-  ProfScope ps(PK_SPECTRUM, st, 0.0, sizeof(T) * static_cast<double>(count) * n * n);
-  jacobi_spectrum_kernel<T, CPLX><<<count, 256, smem, st>>>(mats, n, out, sweeps_used);
-  TG_CHECK_LAUNCH();
-  count_launch();
-}
-
 void spectrum_distance(const double* a, const double* c, int count, int n, double* sig,
                        cudaStream_t st) {
   if (count <= 0) return;
@@ -2998,35 +2858,19 @@ void upper_to_rh(const T* acm, int64_t lda, int64_t k, T* out, cudaStream_t st) 
   count_launch();
 }
 
-template <typename T>
-int jacobi_svd_max_k() {
-  // A and W (re [, im]) plus norms / positions must fit in 227 KB of smem
-  return is_cplx<T>::value ? 84 : 119;
-}
-
-template <typename T>
-void jacobi_svd(const T* A, int64_t k, T* U, double* S, T* W, cudaStream_t st, const T* Winit) {
-  constexpr bool CPLX = is_cplx<T>::value;
-  if (k < 1 || k > jacobi_svd_max_k<T>()) fail(TG_E_INPUT, "jacobi_svd: k out of range");
-  const size_t smem = sizeof(double) * ((CPLX ? 4 : 2) * k * k + k) + sizeof(int) * k;
-  ProfScope ps(PK_SOLVER, st, (CPLX ? 4.0 : 1.0) * 10.0 * static_cast<double>(k) * k * k, 0.0);
+void jacobi_svd_complex(const cplx* A, int64_t k, cplx* U, double* S, cplx* W, cudaStream_t st) {
+  const size_t smem = sizeof(double) * (4 * k * k + k) + sizeof(int) * k;
   const int npairs = static_cast<int>((k + 1) / 2);
-  // up to 96 columns: 16 lanes a pair, 3, 4 or 6 rows a lane; up to 160: 32 lanes, 5 rows
-  auto run = [&](auto kernel, int lanes) {
+  auto run = [&](auto kernel) {
     ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
-    const int threads = static_cast<int>(std::min<int64_t>(1024, (static_cast<int64_t>(npairs) * lanes + 31) / 32 * 32));
-    kernel<<<1, threads, smem, st>>>(A, static_cast<int>(k), U, S, W, Winit);
+    const int threads = static_cast<int>(std::min<int64_t>(1024, (static_cast<int64_t>(npairs) * 16 + 31) / 32 * 32));
+    kernel<<<1, threads, smem, st>>>(A, static_cast<int>(k), U, S, W, nullptr);
   };
   // rows a lane holds: the fewest that cover k (masked rows add exact zeros,
   // so the sums -- and the result -- are those of any larger choice)
-  if (k <= 48)
-    run(jacobi_svd_kernel<T, CPLX, 16, 3>, 16);
-  else if (k <= 64)
-    run(jacobi_svd_kernel<T, CPLX, 16, 4>, 16);
-  else if (k <= 96)
-    run(jacobi_svd_kernel<T, CPLX, 16, 6>, 16);
-  else
-    run(jacobi_svd_kernel<T, CPLX, 32, 5>, 32);
+  if (k <= 48) run(jacobi_svd_kernel<cplx, true, 16, 3>);
+  else if (k <= 64) run(jacobi_svd_kernel<cplx, true, 16, 4>);
+  else run(jacobi_svd_kernel<cplx, true, 16, 6>);
   TG_CHECK_LAUNCH();
   count_launch();
 }
@@ -3069,8 +2913,6 @@ void chol_rinv(const T* parts, int nparts, int64_t k, int64_t n, int shift, T* R
   template void chol_rinv<T>(const T*, int, int64_t, int64_t, int, T*, int*, cudaStream_t);        \
   template void counter_normal<T>(T*, int64_t, int64_t, uint64_t, uint64_t, cudaStream_t);       \
   template void upper_to_rh<T>(const T*, int64_t, int64_t, T*, cudaStream_t);                    \
-  template int jacobi_svd_max_k<T>();                                                            \
-  template void jacobi_svd<T>(const T*, int64_t, T*, double*, T*, cudaStream_t, const T*);       \
   template void gemm<T>(const T*, const T*, T*, const GemmDesc&, cudaStream_t);                  \
   template void gemm_group<T>(const GroupItem*, int, cudaStream_t);                             \
   template bool gemm_specialised<T>(const GemmDesc&);                                            \
@@ -3084,7 +2926,6 @@ void chol_rinv(const T* parts, int nparts, int64_t k, int64_t n, int shift, T* R
                               cudaStream_t);                                                     \
   template void identity<T>(T*, int64_t, cudaStream_t);                                          \
   template void ritz_residual<T>(const T*, const T*, const double*, int64_t, int, double*, cudaStream_t); \
-  template void batched_spectrum<T>(const T* const*, int, int, double*, int*, cudaStream_t);     \
   template void scale<T>(T*, int64_t, double, cudaStream_t);                                     \
   template void axpy<T>(T*, const T*, double, int64_t, cudaStream_t);                            \
   template void scale_leg<T>(T*, int64_t, int64_t, int64_t, const double*, cudaStream_t);

@@ -166,8 +166,7 @@ void identity(T* out, int64_t e, cudaStream_t st);
 // Jacobi (one CTA per matrix, matrix resident in shared memory).  Values are
 // written descending to out[b*n + i].  n <= 160 (real), 112 (complex).
 template <typename T>
-void batched_spectrum(const T* const* mats, int count, int n, double* out, int* sweeps_used,
-                      cudaStream_t st);
+void batched_spectrum(const T* const* mats, int count, int n, double* out, cudaStream_t st);
 
 // sig[b] = || a[b*n : (b+1)*n] - c[b*n : (b+1)*n] ||_2
 void spectrum_distance(const double* a, const double* c, int count, int n, double* sig,
@@ -186,15 +185,14 @@ void counter_normal(T* out_colmajor, int64_t rows, int64_t cols, uint64_t seed, 
 template <typename T>
 void upper_to_rh(const T* acm, int64_t lda, int64_t k, T* out, cudaStream_t st);
 
-// SVD of one row-major k x k matrix by one-sided Jacobi with accumulated
-// right vectors, in one CTA with A and W resident in shared memory:
-// A W = U S, singular values descending.  U, W written row-major (k x k,
-// column j = j-th singular vector), S (k).  k <= jacobi_svd_max_k<T>().
-// With Winit the accumulated rotations start from Winit instead of the
-// identity: pass A = B Winit (Winit unitary) and the result is the SVD of B,
-// B W = U S -- a warm start when Winit already nearly diagonalises B.
+// SVD of one row-major k x k matrix by one-sided Jacobi (jacobi.cu): A W = U S,
+// singular values descending.  U, W written row-major (k x k, column j = j-th
+// singular vector), S (k).  k <= jacobi_svd_max_k<T>().  circle: the order and
+// angles of the randomised projectors, whose results carry every rounding.
 template <typename T>
-void jacobi_svd(const T* A, int64_t k, T* U, double* S, T* W, cudaStream_t st, const T* Winit = nullptr);
+void jacobi_svd(const T* A, int64_t k, T* U, double* S, T* W, bool circle, cudaStream_t st);
+// the circle form of complex matrices (k <= 84): A and W side by side in one CTA
+void jacobi_svd_complex(const cplx* A, int64_t k, cplx* U, double* S, cplx* W, cudaStream_t st);
 template <typename T>
 int jacobi_svd_max_k();
 

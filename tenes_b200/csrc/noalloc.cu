@@ -75,10 +75,9 @@ extern "C" tg_status tg_corner_spectra_noalloc(const void* const* device_mats, i
     TG_CUDA(cudaMemcpyAsync(table, staged, sizeof(void*) * count, cudaMemcpyHostToDevice, st));
     if (is_complex) {
       tg::batched_spectrum<tg::cplx>(reinterpret_cast<const tg::cplx* const*>(table), count, n, device_out,
-                                     nullptr, st);
+                                     st);
     } else {
-      tg::batched_spectrum<double>(reinterpret_cast<const double* const*>(table), count, n, device_out, nullptr,
-                                   st);
+      tg::batched_spectrum<double>(reinterpret_cast<const double* const*>(table), count, n, device_out, st);
     }
     return TG_OK;
   } catch (const tg::Error& e) {

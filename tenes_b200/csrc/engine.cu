@@ -10,6 +10,7 @@
 #include <algorithm>
 #include <cmath>
 #include <complex>
+#include <functional>
 #include <numeric>
 #include <cstring>
 #include <map>
@@ -234,6 +235,7 @@ struct EngineT final : Engine {
     cudaFree(d_ptrs);
     cudaFreeHost(h_ptrs);
     cudaFreeHost(h_sig);
+    if (h_solve) cudaFreeHost(h_solve);
     for (int r = 0; r < kRowStreams; ++r) {
       if (row_st[r]) cudaStreamDestroy(row_st[r]);
       if (ev_join[r]) cudaEventDestroy(ev_join[r]);
@@ -272,10 +274,16 @@ struct EngineT final : Engine {
   // `parallel`, else in order on the current stream.  Tensors that a row
   // creates and that outlive it must be handed to `st` with keep() before
   // they are released, so that their release is ordered after every row.
-  template <typename F>
-  void for_rows(int n, bool parallel, F&& body) {
+  // `step`(r), on the same streams after every body, in turn until it returns
+  // false for each row.
+  template <typename F, typename G>
+  void for_rows(int n, bool parallel, F&& body, G&& step) {
     if (!parallel || n < 2) {
-      for (int r = 0; r < n; ++r) body(r);
+      for (int r = 0; r < n; ++r) {
+        body(r);
+        while (step(r)) {
+        }
+      }
       return;
     }
     const int ns = std::min(n, kRowStreams);
@@ -294,13 +302,26 @@ struct EngineT final : Engine {
         cudaStreamWaitEvent(st, ev_join[s], 0);
       }
     };
+    auto on = [&](int r) {
+      st = row_st[r % ns];
+      slot = 1 + r % ns;
+      cur_row = stagger ? r : -1;
+    };
     try {
       for (int r = 0; r < n; ++r) {
-        st = row_st[r % ns];
-        slot = 1 + r % ns;
-        cur_row = stagger ? r : -1;
+        on(r);
         body(r);
       }
+      std::vector<char> more(static_cast<size_t>(n), 1);
+      for (int left = n; left > 0;)
+        for (int r = 0; r < n; ++r) {
+          if (!more[static_cast<size_t>(r)]) continue;
+          on(r);
+          if (!step(r)) {
+            more[static_cast<size_t>(r)] = 0;
+            --left;
+          }
+        }
     } catch (...) {
       join();
       throw;
@@ -324,9 +345,7 @@ struct EngineT final : Engine {
       if (t.mem) t.mem->st = st;
   }
   // Rows run on their own streams except under the per-kernel profiler,
-  // whose attribution wants one launch at a time.  (Rows with full-SVD
-  // projectors synchronise with the host at every residual check, so they
-  // overlap only with the rows that follow them.)
+  // whose attribution wants one launch at a time.
   bool rows_parallel() const { return !profile_enabled(); }
 
   void upload(DT<T>& t, const double* host) {
@@ -882,117 +901,147 @@ struct EngineT final : Engine {
     return b >= w + 8 ? static_cast<int>(b) : -1;
   }
 
-  // Truncated factors of M (views m = M, mh = M^H, nrow x ncol) as rsvd_run
-  // returns them: Uc (nrow x w) and Vc (ncol x w), row-major, scaled by
-  // 1/sqrt(s), zero past the cut.  Returns false when the dense SVD must be
-  // used (block too small for chi, or no convergence).
-  bool exact_factors(const MV& m, const MV& mh, int64_t nrow, int64_t ncol, DT<T>& Uc, DT<T>& Vc) {
-    const int64_t kmax = std::min(nrow, ncol);
-    const int b = exact_block(kmax);
-    if (b < 1) return false;
-    PrecScope fp64(this, 0);
-    const int w = static_cast<int>(std::min<int64_t>(P.chi, kmax));
-    ++exact_solves;
+  // One such solve, in steps: advance() enqueues the iterations up to the next
+  // residual check and the copies of its results to the host, check() reads
+  // them once the stream has run them.  The rows of a move take these steps in
+  // turn (project_rows), so that one row's kernels run while the host waits
+  // for another's residuals.  Outputs as rsvd_run returns them: Uc (nrow x w)
+  // and Vc (ncol x w), row-major, scaled by 1/sqrt(s), zero past the cut.
+  struct ExactSolve {
+    EngineT* e;
+    DT<T> M;  // nrow x ncol, row-major
+    int64_t nrow, ncol;
+    int key, b, w;
+    double* host;  // page-locked: b singular values, w residuals, the pivot flag
     // Attempt 0 orthonormalises by shifted CholeskyQR.  A matrix of rank below
     // the block (the padded environments of an iTPO, whose single-layer
     // matrices are narrow) can leave a Gram matrix that no shift makes
     // positive: the solve then starts again with Householder QR, which
     // yields orthonormal columns for any panel, before giving up for the
     // dense SVD.
-    for (int attempt = 0; attempt < 2; ++attempt) {
-      const bool householder = attempt == 1;
-      auto orth = [&](DT<T>& X, int64_t n, int passes) {
-        if (householder) orth_cm(X, n, b);
-        else orth_chol(X, n, b, passes);
-      };
-      DT<T> Om({b, ncol}, st);  // column-major ncol x b
+    bool householder = false;
+    int it = 0, next_check = 0, prev_it = 0;
+    double prev_ratio = 0.0;
+    DT<T> Q, Qz, Ur, Wr, Y;
+    DT<double> s;
+    DT<T> Uc, Vc;
+
+    enum State { kRunning, kDone, kFailed };
+
+    ExactSolve(EngineT* e_, const DT<T>& M_, int64_t nrow_, int64_t ncol_, int b_, double* host_)
+        : e(e_), M(M_), nrow(nrow_), ncol(ncol_), key(e_->proj_key), b(b_), host(host_) {
+      w = static_cast<int>(std::min<int64_t>(e->P.chi, std::min(nrow, ncol)));
+      ++e->exact_solves;
+      start();
+    }
+    void orth(DT<T>& X, int64_t n, int passes) {
+      if (householder) e->orth_cm(X, n, b);
+      else e->orth_chol(X, n, b, passes);
+    }
+    void start() {
+      PrecScope fp64(e, 0);
+      const MV m = rm(M.p, nrow, ncol);
+      DT<T> Om({b, ncol}, e->st);  // column-major ncol x b
       int w0 = 0;
-      auto hit = warm_v.find(proj_key);
-      if (proj_key >= 0 && hit != warm_v.end() && hit->second.size() == static_cast<int64_t>(b) * ncol) {
+      auto hit = e->warm_v.find(key);
+      if (key >= 0 && hit != e->warm_v.end() && hit->second.size() == static_cast<int64_t>(b) * ncol) {
         w0 = w;
-        TG_CUDA(cudaMemcpyAsync(Om.p, hit->second.p, sizeof(T) * w0 * ncol, cudaMemcpyDeviceToDevice, st));
+        TG_CUDA(cudaMemcpyAsync(Om.p, hit->second.p, sizeof(T) * w0 * ncol, cudaMemcpyDeviceToDevice, e->st));
       }
-      if (b > w0) counter_normal<T>(Om.p + static_cast<int64_t>(w0) * ncol, ncol, b - w0, P.rsvd_seed, 7, st);
-      DT<T> Q = mm_cm(m, cm(Om.p, ncol, b));  // nrow x b, column-major
-      int next_check = (w0 > 0 || b == kmax) ? 1 : 3;
+      if (b > w0) counter_normal<T>(Om.p + static_cast<int64_t>(w0) * ncol, ncol, b - w0, e->P.rsvd_seed, 7, e->st);
+      Q = e->mm_cm(m, cm(Om.p, ncol, b));  // nrow x b, column-major
+      it = prev_it = 0;
+      prev_ratio = 0.0;
+      next_check = (w0 > 0 || b == std::min(nrow, ncol)) ? 1 : 3;
       orth(Q, nrow, next_check == 1 ? 4 : 2);
-      std::vector<double> hs(static_cast<size_t>(b)), hr(static_cast<size_t>(w));
-      int prev_it = 0;
-      double prev_ratio = 0.0;
-      bool pivot_failed = false;
-      for (int it = 1; it <= kExactMaxIters; ++it) {
-        ++exact_iters;
-        DT<T> Z = mm_cm(mh, cm(Q.p, nrow, b));  // M^H Q: ncol x b
-        if (it < next_check) {
-          orth(Z, ncol, 2);
-          Q = mm_cm(m, cm(Z.p, ncol, b));
-          orth(Q, nrow, it + 1 == next_check ? 4 : 2);
-          continue;
-        }
-        ++exact_checks;
-        DT<T> Qz = clone(Z, st);
-        orth(Qz, ncol, 4);
-        DT<T> Tm = mm_rm(ht(cm(Z.p, ncol, b)), cm(Qz.p, ncol, b));  // Q^H M Qz (b x b row-major)
-        DT<T> Ur({b, b}, st), Wr({b, b}, st);
-        DT<double> s({b}, st);
-        jacobi_svd<T>(Tm.p, b, Ur.p, s.p, Wr.p, false, st);  // T Wr = Ur S
-        DT<T> Y = mm_cm(m, cm(Qz.p, ncol, b));        // M Qz: nrow x b
-        DT<T> MV1 = mm_cm(cm(Y.p, nrow, b), rm(Wr.p, b, b));  // M v_i
-        DT<T> U1 = mm_cm(cm(Q.p, nrow, b), rm(Ur.p, b, b));   // u_i
-        DT<double> r({w}, st);
-        ritz_residual<T>(MV1.p, U1.p, s.p, nrow, w, r.p, st);
-        int pivot_flag = 0;
-        TG_CUDA(cudaMemcpyAsync(hs.data(), s.p, sizeof(double) * b, cudaMemcpyDeviceToHost, st));
-        TG_CUDA(cudaMemcpyAsync(hr.data(), r.p, sizeof(double) * w, cudaMemcpyDeviceToHost, st));
-        TG_CUDA(cudaMemcpyAsync(&pivot_flag, d_flag + slot, sizeof(int), cudaMemcpyDeviceToHost, st));
-        TG_CUDA(cudaStreamSynchronize(st));
-        if (pivot_flag) {  // an orthonormalisation met a non-positive pivot
-          TG_CUDA(cudaMemsetAsync(d_flag + slot, 0, sizeof(int), st));
-          pivot_failed = true;
+      advance();
+    }
+    void advance() {
+      PrecScope fp64(e, 0);
+      const MV m = rm(M.p, nrow, ncol), mh = ht(m);
+      for (++it; it < next_check; ++it) {
+        ++e->exact_iters;
+        DT<T> Z = e->mm_cm(mh, cm(Q.p, nrow, b));  // M^H Q: ncol x b
+        orth(Z, ncol, 2);
+        Q = e->mm_cm(m, cm(Z.p, ncol, b));
+        orth(Q, nrow, it + 1 == next_check ? 4 : 2);
+      }
+      ++e->exact_iters;
+      ++e->exact_checks;
+      DT<T> Z = e->mm_cm(mh, cm(Q.p, nrow, b));
+      Qz = clone(Z, e->st);
+      orth(Qz, ncol, 4);
+      DT<T> Tm = e->mm_rm(ht(cm(Z.p, ncol, b)), cm(Qz.p, ncol, b));  // Q^H M Qz (b x b row-major)
+      Ur = DT<T>({b, b}, e->st);
+      Wr = DT<T>({b, b}, e->st);
+      s = DT<double>({b}, e->st);
+      jacobi_svd<T>(Tm.p, b, Ur.p, s.p, Wr.p, false, e->st);  // T Wr = Ur S
+      Y = e->mm_cm(m, cm(Qz.p, ncol, b));                     // M Qz: nrow x b
+      DT<T> MV1 = e->mm_cm(cm(Y.p, nrow, b), rm(Wr.p, b, b));  // M v_i
+      DT<T> U1 = e->mm_cm(cm(Q.p, nrow, b), rm(Ur.p, b, b));   // u_i
+      DT<double> r({w}, e->st);
+      ritz_residual<T>(MV1.p, U1.p, s.p, nrow, w, r.p, e->st);
+      TG_CUDA(cudaMemcpyAsync(host, s.p, sizeof(double) * b, cudaMemcpyDeviceToHost, e->st));
+      TG_CUDA(cudaMemcpyAsync(host + b, r.p, sizeof(double) * w, cudaMemcpyDeviceToHost, e->st));
+      TG_CUDA(cudaMemcpyAsync(host + b + w, e->d_flag + e->slot, sizeof(int), cudaMemcpyDeviceToHost, e->st));
+    }
+    State check() {
+      TG_CUDA(cudaStreamSynchronize(e->st));
+      PrecScope fp64(e, 0);
+      int pivot_flag;
+      std::memcpy(&pivot_flag, host + b + w, sizeof(int));
+      if (pivot_flag) {  // an orthonormalisation met a non-positive pivot
+        TG_CUDA(cudaMemsetAsync(e->d_flag + e->slot, 0, sizeof(int), e->st));
+        if (householder) return failed();
+        householder = true;
+        start();
+        return kRunning;
+      }
+      // the kept triplets: the truncation rule of ctm.cpp:277-288
+      int cut = w;
+      for (int i = 0; i < w; ++i)
+        if (!(host[i] > e->P.inverse_projector_cut * host[0])) {
+          cut = i;
           break;
         }
-        // the kept triplets: the truncation rule of ctm.cpp:277-288
-        int cut = w;
-        for (int i = 0; i < w; ++i)
-          if (!(hs[static_cast<size_t>(i)] > P.inverse_projector_cut * hs[0])) {
-            cut = i;
-            break;
-          }
-        double worst = 0.0;
-        for (int i = 0; i < cut; ++i) worst = std::max(worst, hr[static_cast<size_t>(i)]);
-        const double ratio = hs[0] > 0.0 ? worst / (kExactTol * hs[0]) : 0.0;
-        if (ratio <= 1.0 || b == kmax) {
-          DT<T> U = mm_rm(cm(Q.p, nrow, b), rm(Ur.p, b, b));   // nrow x b row-major
-          DT<T> V = mm_rm(cm(Qz.p, ncol, b), rm(Wr.p, b, b));  // ncol x b row-major
-          DT<double> sinv({w}, st);
-          truncation(s.p, b, P.chi, P.inverse_projector_cut, sinv.p, w, d_cut + slot, st);
-          Uc = DT<T>({nrow, w}, st);
-          scale_cols<T>(U.p, b, nrow, w, sinv.p, false, Uc.p, st);
-          Vc = DT<T>({ncol, w}, st);
-          scale_cols<T>(V.p, b, ncol, w, sinv.p, false, Vc.p, st);
-          if (proj_key >= 0) warm_v[proj_key] = mm_cm(cm(Qz.p, ncol, b), rm(Wr.p, b, b));
-          return true;
-        }
-        // a stalled decay (a flat spectrum at the block edge): the dense SVD
-        if (prev_it > 0 && it > 12 && ratio > 0.5 * prev_ratio) break;
-        // iterations to the next check, from the decay seen between the last two
-        int gap = 3;
-        if (prev_it > 0 && ratio < prev_ratio) {
-          const double f = std::pow(ratio / prev_ratio, 1.0 / (it - prev_it));
-          gap = static_cast<int>(std::ceil(std::log(ratio) / -std::log(f)));
-          gap = std::min(16, std::max(1, gap));
-        }
-        prev_it = it;
-        prev_ratio = ratio;
-        next_check = it + gap;
-        Q = std::move(Y);
-        orth(Q, nrow, next_check == it + 1 ? 4 : 2);
+      double worst = 0.0;
+      for (int i = 0; i < cut; ++i) worst = std::max(worst, host[b + i]);
+      const double ratio = host[0] > 0.0 ? worst / (kExactTol * host[0]) : 0.0;
+      if (ratio <= 1.0 || b == std::min(nrow, ncol)) {
+        DT<T> U = e->mm_rm(cm(Q.p, nrow, b), rm(Ur.p, b, b));   // nrow x b row-major
+        DT<T> V = e->mm_rm(cm(Qz.p, ncol, b), rm(Wr.p, b, b));  // ncol x b row-major
+        DT<double> sinv({w}, e->st);
+        truncation(s.p, b, e->P.chi, e->P.inverse_projector_cut, sinv.p, w, e->d_cut + e->slot, e->st);
+        Uc = DT<T>({nrow, w}, e->st);
+        scale_cols<T>(U.p, b, nrow, w, sinv.p, false, Uc.p, e->st);
+        Vc = DT<T>({ncol, w}, e->st);
+        scale_cols<T>(V.p, b, ncol, w, sinv.p, false, Vc.p, e->st);
+        if (key >= 0) e->warm_v[key] = e->mm_cm(cm(Qz.p, ncol, b), rm(Wr.p, b, b));
+        return kDone;
       }
-      if (!pivot_failed) break;
+      // a stalled decay (a flat spectrum at the block edge), or too many iterations: the dense SVD
+      if (prev_it > 0 && it > 12 && ratio > 0.5 * prev_ratio) return failed();
+      // iterations to the next check, from the decay seen between the last two
+      int gap = 3;
+      if (prev_it > 0 && ratio < prev_ratio) {
+        const double f = std::pow(ratio / prev_ratio, 1.0 / (it - prev_it));
+        gap = static_cast<int>(std::ceil(std::log(ratio) / -std::log(f)));
+        gap = std::min(16, std::max(1, gap));
+      }
+      if (it + gap > kExactMaxIters) return failed();
+      prev_it = it;
+      prev_ratio = ratio;
+      next_check = it + gap;
+      Q = std::move(Y);
+      orth(Q, nrow, next_check == it + 1 ? 4 : 2);
+      advance();
+      return kRunning;
     }
-    ++exact_dense;
-    return false;
-  }
+    State failed() {
+      ++e->exact_dense;
+      return kFailed;
+    }
+  };
 
   // The SVD of a strongly rectangular M (nrow x ncol, row-major; the long
   // side at least 4 times the short one k, and k within the one-CTA Jacobi
@@ -1030,17 +1079,9 @@ struct EngineT final : Engine {
     return true;
   }
 
-  // Truncated projectors from M (nrow x ncol, consumed):
+  // Truncated factors from the dense SVD of M (nrow x ncol, consumed):
   // U_c (nrow x w), VT_c (w x ncol) scaled by 1/sqrt(s), w = min(k, chi)
-  void truncated_factors(DT<T>& M, int64_t nrow, int64_t ncol, DT<T>& Uc, DT<T>& VTc) {
-    if (P.svd_solver == 0) {
-      const MV m = rm(M.p, nrow, ncol);
-      DT<T> Vc;
-      if (exact_factors(m, ht(m), nrow, ncol, Uc, Vc)) {
-        VTc = transpose<T>(Vc, {1, 0}, st, true);  // VT_c = V_c^H (w x ncol)
-        return;
-      }
-    }
+  void dense_factors(DT<T>& M, int64_t nrow, int64_t ncol, DT<T>& Uc, DT<T>& VTc) {
     DT<T> U, VT;
     DT<double> s;
     if (!small_side_svd(M, nrow, ncol, U, s, VT)) svd(M, nrow, ncol, U, s, VT);
@@ -1054,10 +1095,76 @@ struct EngineT final : Engine {
     scale_rows<T>(VT.p, ncol, ncol, w, sinv.p, false, VTc.p, st);
   }
 
+  // The projectors of one row: finished where `solve` is null, else waiting
+  // for its factors, from which `finish` (given Uc and VTc) makes them.
+  struct ProjRow {
+    DT<T> PU, PL;
+    std::unique_ptr<ExactSolve> solve;
+    std::function<void(ProjRow&, const DT<T>&, const DT<T>&)> finish;
+    double* host = nullptr;
+  };
+  // U_c and VT_c of M (nrow x ncol, consumed), then row.finish: at once from
+  // the dense SVD, or by an ExactSolve
+  void factor_row(ProjRow& row, DT<T>& M, int64_t nrow, int64_t ncol) {
+    const int b = P.svd_solver == 0 ? exact_block(std::min(nrow, ncol)) : -1;
+    if (b > 0) {
+      row.solve = std::make_unique<ExactSolve>(this, M, nrow, ncol, b, row.host);
+      return;
+    }
+    DT<T> Uc, VTc;
+    dense_factors(M, nrow, ncol, Uc, VTc);
+    row.finish(row, Uc, VTc);
+  }
+  void step_row(ProjRow& row) {
+    ExactSolve& x = *row.solve;
+    const typename ExactSolve::State state = x.check();
+    if (state == ExactSolve::kRunning) return;
+    if (state == ExactSolve::kDone) {
+      row.finish(row, x.Uc, transpose<T>(x.Vc, {1, 0}, st, true));  // VT_c = V_c^H (w x ncol)
+    } else {
+      DT<T> M = x.M, Uc, VTc;
+      dense_factors(M, x.nrow, x.ncol, Uc, VTc);
+      row.finish(row, Uc, VTc);
+    }
+    row.solve.reset();
+  }
+
+  // The projectors of every row of a move, begin(r, row) making row r's or
+  // starting its solve; the solves then take their steps in turn, each on its
+  // row's stream.
+  static constexpr int kSolveHost = 256;  // doubles of a solve's host buffer (b + w + 1 <= 193)
+  double* h_solve = nullptr;
+  int h_solve_rows = 0;
+  template <typename F>
+  void project_rows(int n, std::vector<DT<T>>& PUs, std::vector<DT<T>>& PLs, F&& begin) {
+    if (P.svd_solver == 0 && n > h_solve_rows) {
+      TG_CUDA(cudaStreamSynchronize(st));
+      if (h_solve) cudaFreeHost(h_solve);
+      h_solve = nullptr;
+      TG_CUDA(cudaMallocHost(&h_solve, sizeof(double) * kSolveHost * static_cast<size_t>(n)));
+      h_solve_rows = n;
+    }
+    std::vector<ProjRow> rows(static_cast<size_t>(n));
+    for_rows(
+        n, rows_parallel(),
+        [&](int r) {
+          rows[static_cast<size_t>(r)].host = h_solve + static_cast<ptrdiff_t>(kSolveHost) * r;
+          begin(r, rows[static_cast<size_t>(r)]);
+        },
+        [&](int r) {
+          ProjRow& row = rows[static_cast<size_t>(r)];
+          if (row.solve) step_row(row);
+          return row.solve != nullptr;
+        });
+    for (int r = 0; r < n; ++r) {
+      PUs[static_cast<size_t>(r)] = rows[static_cast<size_t>(r)].PU;
+      PLs[static_cast<size_t>(r)] = rows[static_cast<size_t>(r)].PL;
+    }
+  }
+
   // Calc_projector_left_block (ctm.cpp:174-318)
   void proj_left_block(const DT<T>& C1, const DT<T>& C4, const DT<T>& eT1, const DT<T>& eT6,
-                       const DT<T>& eT7, const DT<T>& eT8, const DT<T>& T1, const DT<T>& T4, DT<T>& PU,
-                       DT<T>& PL) {
+                       const DT<T>& eT7, const DT<T>& eT8, const DT<T>& T1, const DT<T>& T4, ProjRow& row) {
     const int64_t e12 = eT1.dim(1), e56 = eT6.dim(0), e78 = eT8.dim(0);
     const int64_t t12 = T1.dim(2), t41 = T1.dim(3), t34 = T4.dim(2);
     // the bra's bond dimensions: t.. again, or 1 in the single-layer network of an iTPO
@@ -1085,8 +1192,15 @@ struct EngineT final : Engine {
           lbh.split = &s_lbh.op;
         }
       }
-      DT<T> Uc, Vrow;  // Uc: nrow x w;  PU = LBm * Vc where Vc = (VT_c)^H
-      MV vc{nullptr, 0, 0, 0, 0, false};
+      // PU = tensordot(LB, conj(VT_c), Axes(1,3,5), Axes(1,2,3)).transpose(1,0,2,3)  (ctm.cpp:263-266),
+      // PL = tensordot(LT, conj(U_c), Axes(0,2,4), Axes(0,1,2)).transpose(1,0,2,3), with vc = (VT_c)^H
+      auto close = [=](ProjRow& out, const MV& left, const MV& down, const DT<T>& Uc, const MV& vc) {
+        const int64_t w = Uc.dim(1);
+        out.PU = tr(reshape(mm_rm(down, vc), {t41, e78, b41, w}), {1, 0, 2, 3});
+        MV uc = rm(Uc.p, nrow, w);
+        uc.conj = true;
+        out.PL = tr(reshape(mm_rm(left, uc), {t41, e78, b41, w}), {1, 0, 2, 3});
+      };
       if ((t12 != 1 && t34 != 1) && P.use_rsvd) {
         // cut = min(chi, e78 t41^2, e12 t12^2, e56 t34^2), k = factor * cut (ctm.cpp:242-244;
         // single layer: e78 t41, ..., ctm_single.cpp:200-203)
@@ -1098,26 +1212,22 @@ struct EngineT final : Engine {
           fail(TG_E_INPUT, "rSVD sketch size " + std::to_string(k) + " exceeds " +
                                std::to_string(jacobi_svd_max_k<T>()) +
                                " (lower rsvd_oversampling_factor or set rsvd_oversample_abs)");
+        DT<T> Uc, Vrow;  // Uc: nrow x w, Vrow: ncol x w
         rsvd_factors(lt, lth, lb, lbh, nrow, nmid, ncol, cut, k, Uc, Vrow);
-        vc = rm(Vrow.p, ncol, Vrow.dim(1));
+        MV ltt = tp(lt);
+        ltt.split = lth.split;  // real operands: transpose = conjugate transpose
+        close(row, ltt, lb, Uc, rm(Vrow.p, ncol, Vrow.dim(1)));
       } else {
         DT<T> M = mm_rm(lt, lb);
-        truncated_factors(M, nrow, ncol, Uc, Vrow);  // Vrow = VT_c (w x ncol)
-        vc = ht(rm(Vrow.p, Vrow.dim(0), ncol));
+        row.finish = [=](ProjRow& out, const DT<T>& Uc, const DT<T>& VTc) {  // keeps LTm and LBm
+          close(out, tp(rm(LTm.p, nrow, nmid)), rm(LBm.p, nmid, ncol), Uc, ht(rm(VTc.p, VTc.dim(0), ncol)));
+        };
+        factor_row(row, M, nrow, ncol);
       }
-      const int64_t w = Uc.dim(1);
-      // PU = tensordot(LB, conj(VT_c), Axes(1,3,5), Axes(1,2,3)).transpose(1,0,2,3)  (ctm.cpp:263-266)
-      PU = tr(reshape(mm_rm(lb, vc), {t41, e78, b41, w}), {1, 0, 2, 3});
-      // PL = tensordot(LT, conj(U_c), Axes(0,2,4), Axes(0,1,2)).transpose(1,0,2,3)
-      MV uc = rm(Uc.p, nrow, w);
-      uc.conj = true;
-      MV ltt = tp(lt);
-      ltt.split = lth.split;  // real operands: transpose = conjugate transpose
-      PL = tr(reshape(mm_rm(ltt, uc), {t41, e78, b41, w}), {1, 0, 2, 3});
     } else {
-      PU = DT<T>({e78, 1, 1, e78}, st);
-      identity<T>(PU.p, e78, st);
-      PL = clone(PU, st);
+      row.PU = DT<T>({e78, 1, 1, e78}, st);
+      identity<T>(row.PU.p, e78, st);
+      row.PL = clone(row.PU, st);
     }
   }
 
@@ -1181,7 +1291,7 @@ struct EngineT final : Engine {
   void proj_updown(const DT<T>& C1, const DT<T>& C2, const DT<T>& C3, const DT<T>& C4, const DT<T>& eT1,
                    const DT<T>& eT2, const DT<T>& eT3, const DT<T>& eT4, const DT<T>& eT5, const DT<T>& eT6,
                    const DT<T>& eT7, const DT<T>& eT8, const DT<T>& T1, const DT<T>& T2, const DT<T>& T3,
-                   const DT<T>& T4, DT<T>& PU, DT<T>& PL) {
+                   const DT<T>& T4, ProjRow& row) {
     const int64_t e78 = eT7.dim(1), e34 = eT3.dim(1);
     const int64_t t23 = T2.dim(3), t41 = T4.dim(1);
     if (t41 != 1) {
@@ -1192,25 +1302,24 @@ struct EngineT final : Engine {
       DT<T> RB = td(T3, X, {2, 3, 4}, {3, 1, 6});
       DT<T> LB = block_LB(C4, eT7, eT6, T4);
       if (t23 != 1 && P.use_rsvd) {
-        proj_updown_rsvd(LT, RT, RB, LB, e34, t23, bra(T2).dim(3), e78, t41, bra(T4).dim(1), PU, PL);
+        proj_updown_rsvd(LT, RT, RB, LB, e34, t23, bra(T2).dim(3), e78, t41, bra(T4).dim(1), row.PU, row.PL);
         return;
       }
       DT<T> R1 = td(RT, LT, {0, 3, 4}, {0, 2, 4});
       DT<T> R2 = td(RB, LB, {0, 2, 4}, {1, 3, 5});
       DT<T> M = td(R1, R2, {3, 4, 5}, {3, 4, 5});
       const int64_t nrow = M.dim(0) * M.dim(1) * M.dim(2), ncol = M.dim(3) * M.dim(4) * M.dim(5);
-      DT<T> Uc, VTc;
       const Shape ms = M.sh;
-      truncated_factors(M, nrow, ncol, Uc, VTc);
-      const int64_t w = Uc.dim(1);
-      DT<T> VTc4 = reshape(VTc, {w, ms[3], ms[4], ms[5]});
-      DT<T> Uc4 = reshape(Uc, {ms[0], ms[1], ms[2], w});
-      PU = tr(td(R2, VTc4, {0, 1, 2}, {1, 2, 3}, false, true), {1, 0, 2, 3});
-      PL = tr(td(R1, Uc4, {0, 1, 2}, {0, 1, 2}, false, true), {1, 0, 2, 3});
+      row.finish = [=](ProjRow& out, const DT<T>& Uc, const DT<T>& VTc) {
+        const int64_t w = Uc.dim(1);
+        out.PU = tr(td(R2, reshape(VTc, {w, ms[3], ms[4], ms[5]}), {0, 1, 2}, {1, 2, 3}, false, true), {1, 0, 2, 3});
+        out.PL = tr(td(R1, reshape(Uc, {ms[0], ms[1], ms[2], w}), {0, 1, 2}, {0, 1, 2}, false, true), {1, 0, 2, 3});
+      };
+      factor_row(row, M, nrow, ncol);
     } else {
-      PU = DT<T>({e78, 1, 1, e78}, st);
-      identity<T>(PU.p, e78, st);
-      PL = clone(PU, st);
+      row.PU = DT<T>({e78, 1, 1, e78}, st);
+      identity<T>(row.PU.p, e78, st);
+      row.PL = clone(row.PU, st);
     }
   }
 
@@ -1368,17 +1477,16 @@ struct EngineT final : Engine {
     auto &C1 = C[0], &C2 = C[1], &C3 = C[2], &C4 = C[3];
     auto &eTt = E[0], &eTr = E[1], &eTb = E[2], &eTl = E[3];
     const int LY = lat.LY_noskew;
-    const bool par = rows_parallel();
     if (density) prepare_rotations();  // Ts, before the rows fork
     std::vector<DT<T>> PUs(LY), PLs(LY);
-    for_rows(LY, par, [&](int iy) {
+    project_rows(LY, PUs, PLs, [&](int iy, ProjRow& row) {
       proj_key = (0 * 4096 + ix) * 4096 + iy;
       const int i = lat.index(ix, iy), j = lat.right(i), k = lat.bottom(j), l = lat.left(k);
       if (P.projector_corner)
-        proj_left_block(C1[i], C4[l], eTt[i], eTb[l], eTl[l], eTl[i], mt(i), mt(l), PUs[iy], PLs[iy]);
+        proj_left_block(C1[i], C4[l], eTt[i], eTb[l], eTl[l], eTl[i], mt(i), mt(l), row);
       else
         proj_updown(C1[i], C2[j], C3[k], C4[l], eTt[i], eTt[j], eTr[j], eTr[k], eTb[k], eTb[l], eTl[l], eTl[i],
-                    mt(i), mt(j), mt(k), mt(l), PUs[iy], PLs[iy]);
+                    mt(i), mt(j), mt(k), mt(l), row);
     });
     std::vector<EtJob> jobs;
     for (int iy = 0; iy < LY; ++iy) {
@@ -1405,17 +1513,16 @@ struct EngineT final : Engine {
     auto &C1 = C[0], &C2 = C[1], &C3 = C[2], &C4 = C[3];
     auto &eTt = E[0], &eTr = E[1], &eTb = E[2], &eTl = E[3];
     const int LY = lat.LY_noskew;
-    const bool par = rows_parallel();
     prepare_rotations();  // before the rows fork
     std::vector<DT<T>> PUs(LY), PLs(LY);
-    for_rows(LY, par, [&](int iy) {
+    project_rows(LY, PUs, PLs, [&](int iy, ProjRow& row) {
       proj_key = (1 * 4096 + ix) * 4096 + iy;
       const int k = lat.index(ix, iy), l = lat.left(k), i = lat.top(l), j = lat.right(i);
       if (P.projector_corner)
-        proj_left_block(C3[k], C2[j], eTb[k], eTt[j], eTr[j], eTr[k], rot(k, 0), rot(j, 0), PUs[iy], PLs[iy]);
+        proj_left_block(C3[k], C2[j], eTb[k], eTt[j], eTr[j], eTr[k], rot(k, 0), rot(j, 0), row);
       else
         proj_updown(C3[k], C4[l], C1[i], C2[j], eTb[k], eTb[l], eTl[l], eTl[i], eTt[i], eTt[j], eTr[j], eTr[k],
-                    rot(k, 0), rot(l, 0), rot(i, 0), rot(j, 0), PUs[iy], PLs[iy]);
+                    rot(k, 0), rot(l, 0), rot(i, 0), rot(j, 0), row);
     });
     std::vector<EtJob> jobs;
     for (int iy = 0; iy < LY; ++iy) {
@@ -1442,17 +1549,16 @@ struct EngineT final : Engine {
     auto &C1 = C[0], &C2 = C[1], &C3 = C[2], &C4 = C[3];
     auto &eTt = E[0], &eTr = E[1], &eTb = E[2], &eTl = E[3];
     const int LX = lat.LX_noskew;
-    const bool par = rows_parallel();
     prepare_rotations();
     std::vector<DT<T>> PUs(LX), PLs(LX);
-    for_rows(LX, par, [&](int ix) {
+    project_rows(LX, PUs, PLs, [&](int ix, ProjRow& row) {
       proj_key = (2 * 4096 + iy) * 4096 + ix;
       const int j = lat.index(ix, iy), k = lat.bottom(j), l = lat.left(k), i = lat.top(l);
       if (P.projector_corner)
-        proj_left_block(C2[j], C1[i], eTr[j], eTl[i], eTt[i], eTt[j], rot(j, 1), rot(i, 1), PUs[ix], PLs[ix]);
+        proj_left_block(C2[j], C1[i], eTr[j], eTl[i], eTt[i], eTt[j], rot(j, 1), rot(i, 1), row);
       else
         proj_updown(C2[j], C3[k], C4[l], C1[i], eTr[j], eTr[k], eTb[k], eTb[l], eTl[l], eTl[i], eTt[i], eTt[j],
-                    rot(j, 1), rot(k, 1), rot(l, 1), rot(i, 1), PUs[ix], PLs[ix]);
+                    rot(j, 1), rot(k, 1), rot(l, 1), rot(i, 1), row);
     });
     std::vector<EtJob> jobs;
     for (int ix = 0; ix < LX; ++ix) {
@@ -1479,17 +1585,16 @@ struct EngineT final : Engine {
     auto &C1 = C[0], &C2 = C[1], &C3 = C[2], &C4 = C[3];
     auto &eTt = E[0], &eTr = E[1], &eTb = E[2], &eTl = E[3];
     const int LX = lat.LX_noskew;
-    const bool par = rows_parallel();
     prepare_rotations();
     std::vector<DT<T>> PUs(LX), PLs(LX);
-    for_rows(LX, par, [&](int ix) {
+    project_rows(LX, PUs, PLs, [&](int ix, ProjRow& row) {
       proj_key = (3 * 4096 + iy) * 4096 + ix;
       const int l = lat.index(ix, iy), i = lat.top(l), j = lat.right(i), k = lat.bottom(j);
       if (P.projector_corner)
-        proj_left_block(C4[l], C3[k], eTl[l], eTr[k], eTb[k], eTb[l], rot(l, 2), rot(k, 2), PUs[ix], PLs[ix]);
+        proj_left_block(C4[l], C3[k], eTl[l], eTr[k], eTb[k], eTb[l], rot(l, 2), rot(k, 2), row);
       else
         proj_updown(C4[l], C1[i], C2[j], C3[k], eTl[l], eTl[i], eTt[i], eTt[j], eTr[j], eTr[k], eTb[k], eTb[l],
-                    rot(l, 2), rot(i, 2), rot(j, 2), rot(k, 2), PUs[ix], PLs[ix]);
+                    rot(l, 2), rot(i, 2), rot(j, 2), rot(k, 2), row);
     });
     std::vector<EtJob> jobs;
     for (int ix = 0; ix < LX; ++ix) {

@@ -389,6 +389,12 @@ tg_status tg_gemm_host_complex(int64_t M, int64_t N, int64_t K, const double* A,
  * tests of the kernels; not part of the CTMRG path. */
 tg_status tg_jacobi_host(int64_t n, int is_complex, int circle, const double* A, double* U, double* S, double* W);
 
+/* SVD A = U diag(S) VT of one row-major m x n host matrix by the engine's dense
+ * solver of small projector matrices (k = min(m, n); (re, im) pairs when
+ * is_complex).  TG_E_RUNTIME when A is not finite.  For tests of the kernels;
+ * not part of the CTMRG path. */
+tg_status tg_svd_host(int64_t m, int64_t n, int is_complex, const double* A, double* U, double* S, double* VT);
+
 /* Orthonormal basis of the span of a real column-major n x k host panel Y
  * (in place) by the engine's shifted CholeskyQR: `passes` passes, the first
  * two shifted, a perturbation of relative size 1e-14 after the first, all in

@@ -402,6 +402,47 @@ extern "C" tg_status tg_jacobi_host(int64_t n, int is_complex, int circle, const
   });
 }
 
+namespace {
+template <typename T>
+int svd_host(int64_t m, int64_t n, const double* A, double* U, double* S, double* VT) {
+  const int64_t k = std::min(m, n);
+  cudaStream_t st;
+  TG_CUDA(cudaStreamCreate(&st));
+  T* d = nullptr;  // A, U, VT
+  double* s = nullptr;
+  int* info = nullptr;
+  TG_CUDA(cudaMalloc(&d, sizeof(T) * (m * n + m * k + k * n)));
+  TG_CUDA(cudaMalloc(&s, sizeof(double) * k));
+  TG_CUDA(cudaMalloc(&info, sizeof(int)));
+  TG_CUDA(cudaMemsetAsync(info, 0, sizeof(int), st));
+  TG_CUDA(cudaMemcpyAsync(d, A, sizeof(T) * m * n, cudaMemcpyHostToDevice, st));
+  tg::dense_svd<T>(d, m, n, d + m * n, s, d + m * n + m * k, info, st);
+  int bad = 0;
+  TG_CUDA(cudaMemcpyAsync(U, d + m * n, sizeof(T) * m * k, cudaMemcpyDeviceToHost, st));
+  TG_CUDA(cudaMemcpyAsync(VT, d + m * n + m * k, sizeof(T) * k * n, cudaMemcpyDeviceToHost, st));
+  TG_CUDA(cudaMemcpyAsync(S, s, sizeof(double) * k, cudaMemcpyDeviceToHost, st));
+  TG_CUDA(cudaMemcpyAsync(&bad, info, sizeof(int), cudaMemcpyDeviceToHost, st));
+  TG_CUDA(cudaStreamSynchronize(st));
+  cudaFree(d);
+  cudaFree(s);
+  cudaFree(info);
+  cudaStreamDestroy(st);
+  return bad;
+}
+}  // namespace
+
+extern "C" tg_status tg_svd_host(int64_t m, int64_t n, int is_complex, const double* A, double* U, double* S,
+                                 double* VT) {
+  return guard([&] {
+    if (!A || !U || !S || !VT) tg::fail(TG_E_INPUT, "bad svd arguments");
+    if (m < 1 || n < 1 ||
+        !(is_complex ? tg::dense_svd_supported<tg::cplx>(m, n) : tg::dense_svd_supported<double>(m, n)))
+      tg::fail(TG_E_INPUT, "svd: unsupported shape");
+    if (is_complex ? svd_host<tg::cplx>(m, n, A, U, S, VT) : svd_host<double>(m, n, A, U, S, VT))
+      tg::fail(TG_E_RUNTIME, "svd: the matrix holds a value that is not finite");
+  });
+}
+
 extern "C" tg_status tg_gemm_group_host(int n, const int64_t* mnk, const int* flags, int is_complex,
                                         const double* A, const double* B, double* C) {
   return guard([&] {

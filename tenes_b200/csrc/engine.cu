@@ -538,7 +538,7 @@ struct EngineT final : Engine {
     for (int i = 0; i < n; ++i)
       if (h[static_cast<size_t>(i)] != 0) {
         TG_CUDA(cudaMemsetAsync(d_info, 0, sizeof(int) * n, st));
-        fail(TG_E_RUNTIME, "cuSOLVER factorisation failed, info = " + std::to_string(h[static_cast<size_t>(i)]));
+        fail(TG_E_RUNTIME, "a factorisation failed, info = " + std::to_string(h[static_cast<size_t>(i)]));
       }
   }
 
@@ -1084,8 +1084,19 @@ struct EngineT final : Engine {
   void dense_factors(DT<T>& M, int64_t nrow, int64_t ncol, DT<T>& Uc, DT<T>& VTc) {
     DT<T> U, VT;
     DT<double> s;
-    if (!small_side_svd(M, nrow, ncol, U, s, VT)) svd(M, nrow, ncol, U, s, VT);
     const int64_t k = std::min(nrow, ncol);
+    if (!small_side_svd(M, nrow, ncol, U, s, VT)) {
+      // the up/down projectors stay with gesvd: R1 R2^T squares the spectrum, and LAPACK-like solvers
+      // return its noise values at 1e-16, below the cut, where the Jacobi's come out at up to 1e-12
+      if (P.svd_solver == 0 && P.projector_corner && dense_svd_supported<T>(nrow, ncol)) {
+        U = DT<T>({nrow, k}, st);
+        s = DT<double>({k}, st);
+        VT = DT<T>({k, ncol}, st);
+        dense_svd<T>(M.p, nrow, ncol, U.p, s.p, VT.p, info_slot(), st);
+      } else {
+        svd(M, nrow, ncol, U, s, VT);
+      }
+    }
     const int w = static_cast<int>(std::min<int64_t>(k, P.chi));
     DT<double> sinv({w}, st);
     truncation(s.p, k, P.chi, P.inverse_projector_cut, sinv.p, w, d_cut + slot, st);

@@ -196,6 +196,17 @@ void jacobi_svd_complex(const cplx* A, int64_t k, cplx* U, double* S, cplx* W, c
 template <typename T>
 int jacobi_svd_max_k();
 
+// SVD of M (nrow x ncol, row-major) in one CTA each for a Householder QR with
+// sorted columns and the Jacobi of R^H (dense_svd.cu): M = U diag(S) VT, U
+// (nrow x k), S (k, descending), VT (k x ncol), row-major, k = min(nrow, ncol).
+// *info (device, may be null) is set to 1 when M holds a value that is not
+// finite.  dense_svd_supported: k <= jacobi_svd_max_k and the matrix in one
+// SM's shared memory, at most 256 on the long side.
+template <typename T>
+bool dense_svd_supported(int64_t nrow, int64_t ncol);
+template <typename T>
+void dense_svd(const T* M, int64_t nrow, int64_t ncol, T* U, double* S, T* VT, int* info, cudaStream_t st);
+
 // x[i] += scale * u_i, u_i counter-based uniform numbers of mean 0 and
 // variance 1 (key derived from `stream`; complex entries get independent real
 // and imaginary parts)

@@ -218,6 +218,50 @@ __global__ void __launch_bounds__(SK_THREADS, 2) skinny_kernel(SkinnyParams p) {
 #undef SKT
 }
 
+// The same product with K, n <= 8 (an operator on a tensor's physical leg, a
+// small bond on a window's boundary): no tile to reuse, one pass over Big and
+// C, a row a thread, the small operand in shared memory.  The streaming kernel
+// pays its stage's barriers for a few hundred bytes there: 6.5e6 rows with
+// K = n = 2 took it 764 us, 1.1 TB/s of 4.8 possible on this many bytes.
+template <int KM, int NM>
+__global__ void __launch_bounds__(256) tiny_kernel(SkinnyParams p) {
+  __shared__ double S[KM * NM];
+  for (int idx = threadIdx.x; idx < KM * NM; idx += 256) {
+    const int k = idx / NM, j = idx % NM;
+    S[idx] = (k < p.K && j < p.n) ? p.small[k * p.ssk + j * p.ssn] : 0.0;
+  }
+  __syncthreads();
+  for (int64_t r = blockIdx.x * int64_t(256) + threadIdx.x; r < p.rows; r += int64_t(256) * gridDim.x) {
+    const double* src = p.big + r * p.sr;
+    double x[KM];
+    if (KM == 2 && p.pairs) {  // both values of the row in one 16-byte load
+      const double2 v = *reinterpret_cast<const double2*>(src);
+      x[0] = v.x;
+      x[KM - 1] = v.y;
+    } else {
+#pragma unroll
+      for (int k = 0; k < KM; ++k) x[k] = k < p.K ? src[k * p.sk] : 0.0;
+    }
+    double* dst = p.C + r * p.scr;
+#pragma unroll
+    for (int j = 0; j < NM; ++j) {
+      if (j >= p.n) break;
+      double v = 0.0;
+#pragma unroll
+      for (int k = 0; k < KM; ++k) v = fma(x[k], S[k * NM + j], v);
+      dst[j * p.scn] = p.accumulate ? dst[j * p.scn] + v : v;
+    }
+  }
+}
+
+template <int KM>
+void launch_tiny(const SkinnyParams& p, cudaStream_t st) {
+  const unsigned grid = static_cast<unsigned>(std::min<int64_t>((p.rows + 255) / 256, 148 * 16));
+  if (p.n <= 2) tiny_kernel<KM, 2><<<grid, 256, 0, st>>>(p);
+  else if (p.n <= 4) tiny_kernel<KM, 4><<<grid, 256, 0, st>>>(p);
+  else tiny_kernel<KM, 8><<<grid, 256, 0, st>>>(p);
+}
+
 size_t skinny_smem(int K, int n, bool kmajor, int stages) {
   const int K4 = (K + 3) & ~3, n8 = (n + 7) & ~7;
   const size_t stage = kmajor ? static_cast<size_t>(K4) * SK_LDR : static_cast<size_t>(SK_R) * sk_ld(K4);
@@ -287,6 +331,18 @@ bool gemm_skinny(const double* A, const double* B, double* C, const GemmDesc& d,
     return false;
   }
   if ((p.sr != 1 && p.sk != 1) || (p.scr != 1 && p.scn != 1)) return false;
+  if (p.K <= 8 && p.n <= 8) {
+    // a row's two values side by side on a 16-byte boundary
+    p.pairs = p.K == 2 && p.sk == 1 && p.sr % 2 == 0 && reinterpret_cast<uintptr_t>(p.big) % 16 == 0;
+    ProfScope ps(PK_GEMM, st, 2.0 * static_cast<double>(d.M) * d.N * d.K,
+                 sizeof(double) * static_cast<double>(d.M * d.K + d.K * d.N + d.M * d.N));
+    if (p.K <= 2) launch_tiny<2>(p, st);
+    else if (p.K <= 4) launch_tiny<4>(p, st);
+    else launch_tiny<8>(p, st);
+    TG_CHECK_LAUNCH();
+    count_launch();
+    return true;
+  }
   const bool kmajor = p.sk != 1;
   // 16-byte copies: every unit-stride run of Big starts 16-byte aligned
   const int64_t lead = kmajor ? p.sk : p.sr;

@@ -11,7 +11,9 @@ from tenes_b200._lib import check, dptr
 pytestmark = pytest.mark.gpu
 
 SHAPES = [(1, 1, 1), (5, 3, 2), (16, 16, 32), (17, 25, 33), (33, 17, 31), (47, 31, 65), (40, 40, 40), (100, 50, 128),
-          (243, 37, 243), (512, 42, 512), (64, 64, 4097), (7, 300, 1000), (48, 48, 1200), (17, 2000, 97)]
+          (243, 37, 243), (512, 42, 512), (64, 64, 4097), (7, 300, 1000), (48, 48, 1200), (17, 2000, 97),
+          # one long side, the others at most 8: a row a thread (skinny.cu)
+          (2048, 1, 1), (2500, 2, 2), (3, 5000, 8), (4097, 8, 5), (4, 70001, 3)]
 
 
 @pytest.mark.parametrize("M,N,K", SHAPES)

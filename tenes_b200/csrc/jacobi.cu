@@ -33,6 +33,7 @@
 #include <type_traits>
 
 #include "kernels.cuh"
+#include "rotation.cuh"
 
 namespace tg {
 namespace {
@@ -163,8 +164,7 @@ __device__ __forceinline__ double re_of(double x) { return x; }
 __device__ __forceinline__ double re_of(cplx x) { return x.x; }
 __device__ __forceinline__ double im_of(cplx x) { return x.y; }
 
-// The rotation of columns with squared norms al, be and |inner product| g:
-// t = tan, the smaller root of t^2 + 2 zeta t = 1 with zeta = (be - al) / 2g.
+// rotation_angle in double precision
 __device__ __forceinline__ void angle_double(double al, double be, double g, double& t, double& c, double& s) {
   const double tau = be - al;
   const double w = fma(tau, tau, 4.0 * g * g);
@@ -174,24 +174,6 @@ __device__ __forceinline__ void angle_double(double al, double be, double g, dou
   c = rsqrt(fma(t, t, 1.0));
   s = c * t;
 }
-// the same from single-precision t
-__device__ __forceinline__ void angle(double al, double be, double g, double& t, double& c, double& s) {
-  const double tau = be - al, g2 = 2.0 * g;
-  // both scaled by the power of two that takes the larger one into [1, 2)
-  const int ha = __double2hiint(fabs(tau)), hg = __double2hiint(g2);
-  const int e = min((ha > hg ? ha : hg) & 0x7ff00000, 0x7fd00000);
-  const double scale = __hiloint2double(0x7fe00000 - e, 0);
-  const float a = __double2float_rn(fabs(tau) * scale), b = __double2float_rn(g2 * scale);
-  const float w = fmaf(a, a, b * b);
-  const float tf = __fdividef(b, a + w * rsqrtf(w));
-  const float cf = rsqrtf(fmaf(tf, tf, 1.0f));
-  t = copysign(static_cast<double>(tf), tau);
-  const double c0 = static_cast<double>(cf), h = fma(t, t, 1.0) * c0;
-  const double err = fma(-h, c0, 1.0);  // 1 - (1 + t^2) c0^2, about 1e-7
-  c = fma(c0 * err, fma(err, 0.375, 0.5), c0);
-  s = c * t;
-}
-
 // (p, q) -> (c p - s b, s p + c b) with b = ph q
 __device__ __forceinline__ void rotate_pair(double c, double s, double phr, double phi, double& pr, double& pi,
                                             double& qr, double& qi) {
@@ -225,8 +207,10 @@ __device__ double block_sum(double a) {
 // order to U, the rotations to `log` (round-major) and {sweeps, position of
 // every column} to `info`.  kSpectrum: the norms, divided by their 2-norm,
 // descending to S, one matrix a CTA (mats[blockIdx.x]).
+// WIDE: more columns than the CTA's lanes can hold; a group takes several pairs
+// of a circle tournament in turn.
 enum JacobiMode { kSpectrum, kSvd, kCircle };
-template <bool CPLX, int LANES, int RPL, int MODE, int THREADS>
+template <bool CPLX, int LANES, int RPL, int MODE, int THREADS, bool WIDE>
 __global__ void __launch_bounds__(THREADS)
     jacobi_kernel(const void* A0, const void* const* mats, int n, void* U0, double* S, Rot<CPLX>* log, int* info) {
   using T = typename std::conditional<CPLX, cplx, double>::type;
@@ -242,7 +226,7 @@ __global__ void __launch_bounds__(THREADS)
   __shared__ int rotated;
   const T* A = static_cast<const T*>(VEC ? A0 : mats[blockIdx.x]);
   S += VEC ? 0 : static_cast<int64_t>(blockIdx.x) * n;
-  const Schedule sch(n, MODE == kCircle);
+  const Schedule sch(n, MODE == kCircle || WIDE);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
   const int g = tid / LANES, gl = tid % LANES;
 
@@ -324,7 +308,7 @@ __global__ void __launch_bounds__(THREADS)
       }
       double t, c, s;
       if constexpr (MODE == kCircle) angle_double(al, be, gabs, t, c, s);
-      else angle(al, be, gabs, t, c, s);
+      else rotation_angle(al, be, gabs, t, c, s);
       al = al - t * gabs;
       be = be + t * gabs;
       const double sph = s * phr, cph = c * phr;  // real: phr = +-1
@@ -368,7 +352,7 @@ __global__ void __launch_bounds__(THREADS)
     if (tid == 0) rotated = 0;
     __syncthreads();
     Rot<CPLX>* out = VEC ? log + static_cast<int64_t>(sweep) * sch.rounds() * sch.groups + g : nullptr;
-    if constexpr (MODE != kCircle) {
+    if constexpr (MODE != kCircle && !WIDE) {
       for (int stage = 0; stage < 2; ++stage) {
         const int rounds = stage == 0 ? sch.rounds0 : sch.rounds1;
         const int p = sch.resident(stage, g);
@@ -400,18 +384,21 @@ __global__ void __launch_bounds__(THREADS)
       }
     }
     for (int r = 0; r < sch.rounds2; ++r) {
-      int p = 0, q = 0;
-      const bool valid = sch.circle(g, r, p, q);
-      if (!valid) p = q = 0;
-      load(p * LD + gl, xp, yp);
-      load(q * LD + gl, xq, yq);
-      double al = nrm[p], be = nrm[q];
-      if (rotate(valid, xp, yp, xq, yq, al, be, out)) {
-        store(p * LD + gl, xp, yp);
-        store(q * LD + gl, xq, yq);
-        if (gl == 0) {
-          nrm[p] = al;
-          nrm[q] = be;
+      // whole warps stay together in the sums: `first` is the same for all
+      for (int first = 0; first < (WIDE ? sch.groups : 1); first += THREADS / LANES) {
+        int p = 0, q = 0;
+        const bool valid = sch.circle(g + first, r, p, q);
+        if (!valid) p = q = 0;
+        load(p * LD + gl, xp, yp);
+        load(q * LD + gl, xq, yq);
+        double al = nrm[p], be = nrm[q];
+        if (rotate(valid, xp, yp, xq, yq, al, be, VEC ? out + first : nullptr)) {
+          store(p * LD + gl, xp, yp);
+          store(q * LD + gl, xq, yq);
+          if (gl == 0) {
+            nrm[p] = al;
+            nrm[q] = be;
+          }
         }
       }
       if (VEC) out += sch.groups;
@@ -561,25 +548,29 @@ void launch_w(const Rot<CPLX>* log, const int* info, int n, bool circle, void* W
   count_launch();
 }
 
-// LANES x RPL covers the rows; 16 lanes a column up to 96 rows (fewer lanes
-// left the chains exposed: 0.93-1.06 ms against 0.74 ms with 8 lanes at 82),
-// 8 lanes above, where 16 would exceed a CTA's threads and registers
+// LANES x RPL covers the rows; 16 lanes a column and a group a pair up to 96
+// columns (with 8 lanes and 16-byte accesses 48 columns took 145 us against
+// 135, 96 columns 556 against 541).  Above, 8 lanes hold a column without
+// spilling in 512 (complex 256) threads, which take the pairs of a round in two
+// or three turns: 162 columns took 18.8 ms spilling with a whole round at once,
+// 6.5 ms so.
+constexpr int kMaxResident = 96;
 template <bool CPLX, int MODE>
 void launch_jacobi(const void* A, const void* const* mats, int count, int n, void* U, double* S, Rot<CPLX>* log,
                    int* info, cudaStream_t st) {
-  const Schedule sch(n, MODE == kCircle);
-  auto go = [&](auto kernel, int lanes, int rows) {
+  auto go = [&](auto kernel, int lanes, int rows, int threads) {
     const size_t smem = sizeof(double) * static_cast<size_t>((CPLX ? 2 : 1) * n * (lanes * rows + 1) + n);
     ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
-    kernel<<<count, (sch.groups * lanes + 31) / 32 * 32, smem, st>>>(A, mats, n, U, S, log, info);
+    const int need = (Schedule(n, MODE == kCircle).groups * lanes + 31) / 32 * 32;
+    kernel<<<count, threads > 0 ? threads : need, smem, st>>>(A, mats, n, U, S, log, info);
   };
-  if (n <= 16) go(jacobi_kernel<CPLX, 16, 1, MODE, 192>, 16, 1);
-  else if (n <= 32) go(jacobi_kernel<CPLX, 16, 2, MODE, 320>, 16, 2);
-  else if (n <= 48) go(jacobi_kernel<CPLX, 16, 3, MODE, 448>, 16, 3);
-  else if (n <= 64) go(jacobi_kernel<CPLX, 16, 4, MODE, 576>, 16, 4);
-  else if (n <= 96) go(jacobi_kernel<CPLX, 16, 6, MODE, 800>, 16, 6);
-  else if constexpr (CPLX) go(jacobi_kernel<CPLX, 8, 15, MODE, 512>, 8, 15);
-  else go(jacobi_kernel<CPLX, 8, 21, MODE, 704>, 8, 21);
+  if (n <= 16) go(jacobi_kernel<CPLX, 16, 1, MODE, 192, false>, 16, 1, 0);
+  else if (n <= 32) go(jacobi_kernel<CPLX, 16, 2, MODE, 320, false>, 16, 2, 0);
+  else if (n <= 48) go(jacobi_kernel<CPLX, 16, 3, MODE, 448, false>, 16, 3, 0);
+  else if (n <= 64) go(jacobi_kernel<CPLX, 16, 4, MODE, 576, false>, 16, 4, 0);
+  else if (n <= kMaxResident) go(jacobi_kernel<CPLX, 16, 6, MODE, 800, false>, 16, 6, 0);
+  else if constexpr (CPLX) go(jacobi_kernel<CPLX, 8, 15, MODE, 256, true>, 8, 15, 256);
+  else go(jacobi_kernel<CPLX, 8, 21, MODE, 512, true>, 8, 21, 512);
   TG_CHECK_LAUNCH();
   count_launch();
 }
@@ -603,7 +594,8 @@ void jacobi_svd(const T* A, int64_t k, T* U, double* S, T* W, bool circle, cudaS
     }
   }
   const int n = static_cast<int>(k);
-  const Schedule sch(n, circle);
+  const bool tournament = circle || n > kMaxResident;  // as the kernel's
+  const Schedule sch(n, tournament);
   const size_t log_bytes = sizeof(Rot<CPLX>) * kJacobiSweeps * static_cast<size_t>(std::max(sch.rounds(), 1) * sch.groups);
   void* buf = nullptr;
   TG_CUDA(cudaMallocAsync(&buf, log_bytes + sizeof(int) * static_cast<size_t>(n + 1), st));
@@ -613,7 +605,7 @@ void jacobi_svd(const T* A, int64_t k, T* U, double* S, T* W, bool circle, cudaS
     if (circle) launch_jacobi<CPLX, kCircle>(A, nullptr, 1, n, U, S, log, info, st);
   }
   if (!circle) launch_jacobi<CPLX, kSvd>(A, nullptr, 1, n, U, S, log, info, st);
-  launch_w<CPLX>(log, info, n, circle, W, st);
+  launch_w<CPLX>(log, info, n, tournament, W, st);
   TG_CUDA(cudaFreeAsync(buf, st));
 }
 

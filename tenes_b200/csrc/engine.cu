@@ -125,6 +125,9 @@ struct EngineT final : Engine {
       for (int l = 0; l < 4; ++l) lat.vdim[i][l] = ld->virtual_dims[4 * i + l];
     }
     lat.check_dims();
+    narrow_bonds = !P.density;
+    for (const auto& v : lat.vdim)
+      for (int d : v) narrow_bonds = narrow_bonds && d <= 2;
     if (P.chi < 1) fail(TG_E_INPUT, "chi must be positive");
     if (P.density) {
       // the single-layer environment starts at the bond dimensions
@@ -274,10 +277,10 @@ struct EngineT final : Engine {
   // `parallel`, else in order on the current stream.  Tensors that a row
   // creates and that outlive it must be handed to `st` with keep() before
   // they are released, so that their release is ordered after every row.
-  // `step`(r), on the same streams after every body, in turn until it returns
-  // false for each row.
+  // `step`(r), on the same streams, repeats until it returns false: after
+  // every body and row by row in turn, or (not in_turn) right after the row's.
   template <typename F, typename G>
-  void for_rows(int n, bool parallel, F&& body, G&& step) {
+  void for_rows(int n, bool parallel, bool in_turn, F&& body, G&& step) {
     if (!parallel || n < 2) {
       for (int r = 0; r < n; ++r) {
         body(r);
@@ -311,6 +314,8 @@ struct EngineT final : Engine {
       for (int r = 0; r < n; ++r) {
         on(r);
         body(r);
+        while (!in_turn && step(r)) {
+        }
       }
       std::vector<char> more(static_cast<size_t>(n), 1);
       for (int left = n; left > 0;)
@@ -882,9 +887,22 @@ struct EngineT final : Engine {
   // columns.  If the residuals are not below the tolerance after
   // kExactMaxIters iterations (a flat spectrum at the block edge), the
   // dense SVD is used instead.
+  // Contexts whose results carry the last bits of a singular vector to more
+  // than nine digits: 3xTF32 products turn one into 1e-7; up/down, complex iTPO
+  // and D = 2 environments hold kept values next to the cut (one-ulp changes of
+  // their inputs move them by up to 1e-7, against 1e-13 elsewhere).  Their
+  // solves keep the rotations' order, the rows one after the other (the
+  // perturbation keys count through them), the checks at fixed places and, D = 2
+  // aside, gesvd for the small matrices.
+  bool narrow_bonds = false;  // every bond dimension at most 2, both layers; set with the lattice
+  bool last_bits() const { return P.mixed || !P.projector_corner || (CPLX && density); }
+  bool keep_order() const { return last_bits() || narrow_bonds; }
   static constexpr double kExactTol = 1e-13;
   static constexpr int kExactMaxIters = 80;
   std::map<int, DT<T>> warm_v;   // right basis (ncol x b, column-major) per projector
+  // iterations the same projector's last solve needed: where the next one
+  // looks first (a check costs as much as three to five iterations)
+  std::map<int, int> iter_hint;
   int proj_key = -1;             // set by the moves before each projector
   int64_t exact_solves = 0, exact_iters = 0, exact_checks = 0, exact_dense = 0;
 
@@ -952,7 +970,9 @@ struct EngineT final : Engine {
       Q = e->mm_cm(m, cm(Om.p, ncol, b));  // nrow x b, column-major
       it = prev_it = 0;
       prev_ratio = 0.0;
-      next_check = (w0 > 0 || b == std::min(nrow, ncol)) ? 1 : 3;
+      auto last = e->iter_hint.find(key);
+      next_check = b == std::min(nrow, ncol) ? 1 : key >= 0 && last != e->iter_hint.end() ? last->second : w0 > 0 ? 2 : 3;
+      if (e->keep_order()) next_check = (w0 > 0 || b == std::min(nrow, ncol)) ? 1 : 3;
       orth(Q, nrow, next_check == 1 ? 4 : 2);
       advance();
     }
@@ -975,7 +995,7 @@ struct EngineT final : Engine {
       Ur = DT<T>({b, b}, e->st);
       Wr = DT<T>({b, b}, e->st);
       s = DT<double>({b}, e->st);
-      jacobi_svd<T>(Tm.p, b, Ur.p, s.p, Wr.p, false, e->st);  // T Wr = Ur S
+      jacobi_svd<T>(Tm.p, b, Ur.p, s.p, Wr.p, e->keep_order(), e->st);  // T Wr = Ur S
       Y = e->mm_cm(m, cm(Qz.p, ncol, b));                     // M Qz: nrow x b
       DT<T> MV1 = e->mm_cm(cm(Y.p, nrow, b), rm(Wr.p, b, b));  // M v_i
       DT<T> U1 = e->mm_cm(cm(Q.p, nrow, b), rm(Ur.p, b, b));   // u_i
@@ -1007,7 +1027,18 @@ struct EngineT final : Engine {
       double worst = 0.0;
       for (int i = 0; i < cut; ++i) worst = std::max(worst, host[b + i]);
       const double ratio = host[0] > 0.0 ? worst / (kExactTol * host[0]) : 0.0;
+      // the residual's decay an iteration: seen between the last two checks, or
+      // expected from the kept and the dropped edge of the block's spectrum
+      double decay = 0.5;
+      if (prev_it > 0 && ratio < prev_ratio) decay = std::pow(ratio / prev_ratio, 1.0 / (it - prev_it));
+      else if (cut > 0 && !e->keep_order()) decay = std::min(0.5, (host[b - 1] / host[cut - 1]) * (host[b - 1] / host[cut - 1]));
       if (ratio <= 1.0 || b == std::min(nrow, ncol)) {
+        if (key >= 0) {  // one or two iterations fewer where the residual shows them to spare
+          int spare = 0;
+          while (spare < 2 && ratio * std::pow(decay, -(spare + 1)) <= 1.0 && decay > 0.0) ++spare;
+          e->iter_hint[key] = std::max(2, it - spare);
+          if (householder) e->iter_hint.erase(key);  // a block beyond the rank: look early, to notice it again
+        }
         DT<T> U = e->mm_rm(cm(Q.p, nrow, b), rm(Ur.p, b, b));   // nrow x b row-major
         DT<T> V = e->mm_rm(cm(Qz.p, ncol, b), rm(Wr.p, b, b));  // ncol x b row-major
         DT<double> sinv({w}, e->st);
@@ -1021,13 +1052,10 @@ struct EngineT final : Engine {
       }
       // a stalled decay (a flat spectrum at the block edge), or too many iterations: the dense SVD
       if (prev_it > 0 && it > 12 && ratio > 0.5 * prev_ratio) return failed();
-      // iterations to the next check, from the decay seen between the last two
+      // iterations to the next check
       int gap = 3;
-      if (prev_it > 0 && ratio < prev_ratio) {
-        const double f = std::pow(ratio / prev_ratio, 1.0 / (it - prev_it));
-        gap = static_cast<int>(std::ceil(std::log(ratio) / -std::log(f)));
-        gap = std::min(16, std::max(1, gap));
-      }
+      if ((prev_it == 0 ? !e->keep_order() : ratio < prev_ratio) && decay > 0.0)
+        gap = std::min(16, std::max(1, static_cast<int>(std::ceil(std::log(ratio) / -std::log(decay)))));
       if (it + gap > kExactMaxIters) return failed();
       prev_it = it;
       prev_ratio = ratio;
@@ -1086,9 +1114,9 @@ struct EngineT final : Engine {
     DT<double> s;
     const int64_t k = std::min(nrow, ncol);
     if (!small_side_svd(M, nrow, ncol, U, s, VT)) {
-      // the up/down projectors stay with gesvd: R1 R2^T squares the spectrum, and LAPACK-like solvers
-      // return its noise values at 1e-16, below the cut, where the Jacobi's come out at up to 1e-12
-      if (P.svd_solver == 0 && P.projector_corner && dense_svd_supported<T>(nrow, ncol)) {
+      // (the up/down projectors' R1 R2^T squares the spectrum: LAPACK-like solvers return its noise
+      // values at 1e-16, below the cut, where the Jacobi's come out at up to 1e-12)
+      if (P.svd_solver == 0 && !last_bits() && dense_svd_supported<T>(nrow, ncol)) {
         U = DT<T>({nrow, k}, st);
         s = DT<double>({k}, st);
         VT = DT<T>({k, ncol}, st);
@@ -1157,7 +1185,7 @@ struct EngineT final : Engine {
     }
     std::vector<ProjRow> rows(static_cast<size_t>(n));
     for_rows(
-        n, rows_parallel(),
+        n, rows_parallel(), !keep_order(),
         [&](int r) {
           rows[static_cast<size_t>(r)].host = h_solve + static_cast<ptrdiff_t>(kSolveHost) * r;
           begin(r, rows[static_cast<size_t>(r)]);

@@ -484,9 +484,9 @@ __global__ void __launch_bounds__(32 * kWRows)
 #pragma unroll
     for (int k = 0; k < SLOTS; ++k) {
       c[k] = 0;
-      if (more && lane + 32 * k < groups) {
+      if (more && lane + 32 * k < groups) {  // an entry without a pair is loaded too (and skipped): no load waits for another
+        rot[k] = next[32 * k];
         c[k] = pairs[at + 32 * k];
-        if (c[k] != 0) rot[k] = next[32 * k];
       }
     }
     next += groups;

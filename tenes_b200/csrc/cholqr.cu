@@ -291,22 +291,28 @@ __global__ void __launch_bounds__(CQ_THREADS, 1)
         ds[i] = (i < k && g > 0.0) ? 1.0 / sqrt(g) : 1.0;
       }
       __syncthreads();
-      for (int e = tid; e < total; e += CQ_THREADS) {
-        const int b = btab[e >> 6], w = e & 63;
-        const int r = (b >> 8) * 8 + (w >> 3), c = (b & 255) * 8 + (w & 7);
+      // a warp a block, two neighbouring entries a lane
+      for (int b = warp; b < nblk; b += CQ_WARPS) {
+        const int bb = btab[b], r = (bb >> 8) * 8 + (lane >> 2), c = (bb & 255) * 8 + 2 * (lane & 3);
+        double2* at = reinterpret_cast<double2*>(Rs + r * ld + c);
+        double2 v = *at;
         if (r < k && c < k) {
-          double v = Rs[r * ld + c] * (ds[r] * ds[c]);
-          if (r == c && pass < shifted) v += shift;
-          Rs[r * ld + c] = v;
+          v.x *= ds[r] * ds[c];
+          if (r == c && pass < shifted) v.x += shift;
         }
+        if (r < k && c + 1 < k) {
+          v.y *= ds[r] * ds[c + 1];
+          if (r == c + 1 && pass < shifted) v.y += shift;
+        }
+        *at = v;
       }
       __syncthreads();
       cholesky_blocked(Rs, kp, ld, dinv, btab, flag);
       // R' and D to the global scratch, read from L2 by the other CTAs (a
       // broadcast from one SM's shared memory would serialise on that SM)
-      for (int e = tid; e < total; e += CQ_THREADS) {
-        const int off = entry(e);
-        scratch[off] = Rs[off];
+      for (int b = warp; b < nblk; b += CQ_WARPS) {
+        const int bb = btab[b], off = ((bb >> 8) * 8 + (lane >> 2)) * ld + (bb & 255) * 8 + 2 * (lane & 3);
+        *reinterpret_cast<double2*>(scratch + off) = *reinterpret_cast<const double2*>(Rs + off);
       }
       for (int i = tid; i < kp; i += CQ_THREADS) scratch[kp * ld + i] = ds[i];
       __threadfence();
@@ -314,10 +320,10 @@ __global__ void __launch_bounds__(CQ_THREADS, 1)
     cluster.sync();
     // ---- 4. R' and D from the scratch (L2 only: the lines change every pass)
     if (rank != 0) {
-#pragma unroll 4
-      for (int e = tid; e < total; e += CQ_THREADS) {
-        const int off = entry(e);
-        Rs[off] = __ldcg(scratch + off);
+#pragma unroll 3
+      for (int b = warp; b < nblk; b += CQ_WARPS) {
+        const int bb = btab[b], off = ((bb >> 8) * 8 + (lane >> 2)) * ld + (bb & 255) * 8 + 2 * (lane & 3);
+        *reinterpret_cast<double2*>(Rs + off) = __ldcg(reinterpret_cast<const double2*>(scratch + off));
       }
       for (int i = tid; i < kp; i += CQ_THREADS) ds[i] = __ldcg(scratch + kp * ld + i);
       __syncthreads();

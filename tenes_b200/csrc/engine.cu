@@ -794,7 +794,7 @@ struct EngineT final : Engine {
       DT<T> G({k, k}, st);
       sum_partials<T>(parts.p, nparts, k * k, G.p, st);
       DT<T> Ri({k, k}, st);
-      chol_rinv<T>(G.p, 1, k, n, pass <= 1 ? 1 : 0, Ri.p, d_flag + slot, st);
+      chol_rinv<T>(G.p, k, n, pass <= 1 ? 1 : 0, Ri.p, d_flag + slot, st);
       Y = mm_cm(cm(Y.p, n, k), rm(Ri.p, k, k));
       if (pass == 0) add_noise<T>(Y.p, n * k, 1e-14 / std::sqrt(static_cast<double>(n)), ++noise_stream, st);
     }

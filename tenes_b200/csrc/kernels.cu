@@ -1820,7 +1820,7 @@ __device__ __forceinline__ cplx shfl_v(cplx v, int src) {
 }
 
 // Inverse Cholesky factor of an equilibrated (optionally shifted) Gram
-// matrix summed from split-K partials, one CTA, blocked by 8: kp = k rounded up to 8,
+// matrix, one CTA, blocked by 8: kp = k rounded up to 8,
 // the padding being the identity.  Cholesky (upper, A' = R'^H R'), three
 // barriers per 8-column block: warp 0 factors the 8 x 8 diagonal block in
 // registers (lane c holds column c, rows exchanged by shuffles), one thread
@@ -1828,39 +1828,40 @@ __device__ __forceinline__ cplx shfl_v(cplx v, int src) {
 // update the trailing triangle.  Then R' is inverted in place, two barriers
 // per block: warp 0 inverts the diagonal block, the column block above it
 // becomes -X[0:j0, 0:j0] R'[0:j0, J] X_JJ.  Rinv = D X as before.  One copy
-// of the matrix lives in shared memory (kp^2 values), plus an 8 x kp panel.
+// of the matrix lives in shared memory (kp (kp + 1) values: the odd pitch keeps
+// the column walks of the inversion off one bank), plus an 8 x kp panel.
 template <typename T, bool CPLX>
-__global__ void __launch_bounds__(512) chol_rinv_blocked_kernel(const T* __restrict__ parts, int nparts, int k,
+__global__ void __launch_bounds__(512) chol_rinv_blocked_kernel(const T* __restrict__ gram, int k,
                                                                  double shift, T* __restrict__ Rinv, int* flag) {
   extern __shared__ __align__(16) unsigned char chol_smem[];
-  const int kp = (k + 7) & ~7, nb = kp / 8;
-  T* A = reinterpret_cast<T*>(chol_smem);  // kp x kp, row-major
-  T* P = A + kp * kp;                      // panel, kp x 8
+  const int kp = (k + 7) & ~7, nb = kp / 8, ld = kp + 1;
+  T* A = reinterpret_cast<T*>(chol_smem);  // kp x kp, row-major, pitch ld
+  T* P = A + kp * ld;                      // panel, kp x 8
   double* d = reinterpret_cast<double*>(P + 8 * kp);
   double* dinv = d + kp;  // 1 / R'_ii
   const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5;
-  const int kk = k * k;
-  for (int idx = tid; idx < kp * kp; idx += nt) {
-    const int r = idx / kp, c = idx - r * kp;
-    T v = (r == c) ? one_of<T>() : zero_of<T>();
-    if (r < k && c < k) {
-      v = zero_of<T>();
-      for (int p = 0; p < nparts; ++p) v = vadd(v, parts[static_cast<int64_t>(p) * kk + r * k + c]);
+  const int nw = nt >> 5;
+  // rows over the warps, columns over the lanes, four rows' loads in flight
+  for (int c = lane; c < kp; c += 32) {
+#pragma unroll 4
+    for (int r = warp; r < kp; r += nw) {
+      T v = (r == c) ? one_of<T>() : zero_of<T>();
+      if (r < k && c < k) v = vadd(zero_of<T>(), gram[r * k + c]);
+      A[r * ld + c] = v;
     }
-    A[idx] = v;
   }
   __syncthreads();
   for (int i = tid; i < kp; i += nt) {
-    const double g = re_of(A[i * kp + i]);
+    const double g = re_of(A[i * ld + i]);
     d[i] = (i < k && g > 0.0) ? 1.0 / sqrt(g) : 1.0;
   }
   __syncthreads();
-  for (int idx = tid; idx < kp * kp; idx += nt) {
-    const int r = idx / kp, c = idx - r * kp;
-    if (r < k && c < k) {
-      T v = mul_real(A[idx], d[r] * d[c]);
+  for (int c = lane; c < k; c += 32) {
+#pragma unroll 4
+    for (int r = warp; r < k; r += nw) {
+      T v = mul_real(A[r * ld + c], d[r] * d[c]);
       if (r == c) v = vadd(v, mul_real(one_of<T>(), shift));
-      A[idx] = v;
+      A[r * ld + c] = v;
     }
   }
   __syncthreads();
@@ -1871,7 +1872,7 @@ __global__ void __launch_bounds__(512) chol_rinv_blocked_kernel(const T* __restr
       const int c = lane & 7;
       T col[8];
 #pragma unroll
-      for (int r = 0; r < 8; ++r) col[r] = (r <= c) ? A[(j0 + r) * kp + j0 + c] : zero_of<T>();
+      for (int r = 0; r < 8; ++r) col[r] = (r <= c) ? A[(j0 + r) * ld + j0 + c] : zero_of<T>();
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         double p = __shfl_sync(0xffffffffu, re_of(col[j]), j);
@@ -1891,33 +1892,44 @@ __global__ void __launch_bounds__(512) chol_rinv_blocked_kernel(const T* __restr
       if (lane < 8) {
 #pragma unroll
         for (int r = 0; r < 8; ++r)
-          if (r <= c) A[(j0 + r) * kp + j0 + c] = col[r];
+          if (r <= c) A[(j0 + r) * ld + j0 + c] = col[r];
       }
     }
     __syncthreads();
     for (int c = j0 + 8 + tid; c < kp; c += nt) {  // block row: solve R'_JJ^H x = a
       T x[8];
 #pragma unroll
-      for (int r = 0; r < 8; ++r) x[r] = A[(j0 + r) * kp + c];
+      for (int r = 0; r < 8; ++r) x[r] = A[(j0 + r) * ld + c];
 #pragma unroll
       for (int r = 0; r < 8; ++r) {
 #pragma unroll
-        for (int m = 0; m < r; ++m) x[r] = vsub(x[r], vmul(conj_of(A[(j0 + m) * kp + j0 + r]), x[m]));
+        for (int m = 0; m < r; ++m) x[r] = vsub(x[r], vmul(conj_of(A[(j0 + m) * ld + j0 + r]), x[m]));
         x[r] = mul_real(x[r], dinv[j0 + r]);
       }
 #pragma unroll
-      for (int r = 0; r < 8; ++r) A[(j0 + r) * kp + c] = x[r];
+      for (int r = 0; r < 8; ++r) A[(j0 + r) * ld + c] = x[r];
     }
     __syncthreads();
-    const int n2 = kp - j0 - 8;
-    for (int idx = tid; idx < n2 * n2; idx += nt) {  // trailing triangle
-      const int r = j0 + 8 + idx / n2, c = j0 + 8 + idx % n2;
-      if (c < r) continue;
-      T acc = zero_of<T>();
+    // trailing triangle in 2 x 2 tiles: half the loads of single elements
+    const int n2 = (kp - j0 - 8) / 2;
+    for (int tr = warp; tr < n2; tr += nw)
+      for (int tc = tr + lane; tc < n2; tc += 32) {
+        const int r = j0 + 8 + 2 * tr, c = j0 + 8 + 2 * tc;
+        T a00 = zero_of<T>(), a01 = a00, a10 = a00, a11 = a00;
 #pragma unroll
-      for (int m = 0; m < 8; ++m) acc = vadd(acc, vmul(conj_of(A[(j0 + m) * kp + r]), A[(j0 + m) * kp + c]));
-      A[r * kp + c] = vsub(A[r * kp + c], acc);
-    }
+        for (int m = 0; m < 8; ++m) {
+          const T* row = A + (j0 + m) * ld;
+          const T r0 = conj_of(row[r]), r1 = conj_of(row[r + 1]), c0 = row[c], c1 = row[c + 1];
+          a00 = vadd(a00, vmul(r0, c0));
+          a01 = vadd(a01, vmul(r0, c1));
+          a10 = vadd(a10, vmul(r1, c0));
+          a11 = vadd(a11, vmul(r1, c1));
+        }
+        A[r * ld + c] = vsub(A[r * ld + c], a00);
+        A[r * ld + c + 1] = vsub(A[r * ld + c + 1], a01);
+        if (tr != tc) A[(r + 1) * ld + c] = vsub(A[(r + 1) * ld + c], a10);
+        A[(r + 1) * ld + c + 1] = vsub(A[(r + 1) * ld + c + 1], a11);
+      }
     __syncthreads();
   }
   // ---- in-place blocked inverse of the upper triangle
@@ -1927,7 +1939,8 @@ __global__ void __launch_bounds__(512) chol_rinv_blocked_kernel(const T* __restr
     for (int idx = tid; idx < j0 * 8; idx += nt) {
       const int i = idx >> 3, c = idx & 7;
       T acc = zero_of<T>();
-      for (int m = i; m < j0; ++m) acc = vadd(acc, vmul(A[i * kp + m], A[m * kp + j0 + c]));
+#pragma unroll 4
+      for (int m = i; m < j0; ++m) acc = vadd(acc, vmul(A[i * ld + m], A[m * ld + j0 + c]));
       P[idx] = acc;
     }
     if (warp == 0) {  // X_JJ = R'_JJ^{-1}: lane c solves R'_JJ x = e_c
@@ -1938,14 +1951,14 @@ __global__ void __launch_bounds__(512) chol_rinv_blocked_kernel(const T* __restr
         T s = (r == c) ? one_of<T>() : zero_of<T>();
 #pragma unroll
         for (int m = r + 1; m < 8; ++m)
-          if (m <= c) s = vsub(s, vmul(A[(j0 + r) * kp + j0 + m], x[m]));
+          if (m <= c) s = vsub(s, vmul(A[(j0 + r) * ld + j0 + m], x[m]));
         x[r] = (r <= c) ? mul_real(s, dinv[j0 + r]) : zero_of<T>();
       }
       __syncwarp();
       if (lane < 8) {
 #pragma unroll
         for (int r = 0; r < 8; ++r)
-          if (r <= c) A[(j0 + r) * kp + j0 + c] = x[r];
+          if (r <= c) A[(j0 + r) * ld + j0 + c] = x[r];
       }
     }
     __syncthreads();
@@ -1955,15 +1968,14 @@ __global__ void __launch_bounds__(512) chol_rinv_blocked_kernel(const T* __restr
       T acc = zero_of<T>();
 #pragma unroll
       for (int m = 0; m < 8; ++m)
-        if (m <= c) acc = vadd(acc, vmul(P[i * 8 + m], A[(j0 + m) * kp + j0 + c]));
-      A[i * kp + j0 + c] = vneg(acc);
+        if (m <= c) acc = vadd(acc, vmul(P[i * 8 + m], A[(j0 + m) * ld + j0 + c]));
+      A[i * ld + j0 + c] = vneg(acc);
     }
     __syncthreads();
   }
-  for (int idx = tid; idx < kk; idx += nt) {  // Rinv = D X (upper)
-    const int r = idx / k, c = idx - r * k;
-    Rinv[idx] = (c >= r) ? mul_real(A[r * kp + c], d[r]) : zero_of<T>();
-  }
+  for (int c = lane; c < k; c += 32)  // Rinv = D X (upper)
+#pragma unroll 4
+    for (int r = warp; r < k; r += nw) Rinv[r * k + c] = (c >= r) ? mul_real(A[r * ld + c], d[r]) : zero_of<T>();
 }
 
 __global__ void spectrum_distance_kernel(const double* a, const double* c, int count, int n,
@@ -2891,18 +2903,18 @@ void sum_partials(const T* parts, int nparts, int64_t len, T* out, cudaStream_t 
 }
 
 template <typename T>
-void chol_rinv(const T* parts, int nparts, int64_t k, int64_t n, int shift, T* Rinv, int* flag, cudaStream_t st) {
+void chol_rinv(const T* gram, int64_t k, int64_t n, int shift, T* Rinv, int* flag, cudaStream_t st) {
   constexpr bool CPLX = is_cplx<T>::value;
   if (k < 1 || k > jacobi_svd_max_k<T>()) fail(TG_E_INPUT, "chol_rinv: k out of range");
   const int64_t kp = (k + 7) / 8 * 8;
-  const size_t smem = sizeof(T) * static_cast<size_t>(kp * kp + 8 * kp) + sizeof(double) * static_cast<size_t>(2 * kp);
+  const size_t smem = sizeof(T) * static_cast<size_t>(kp * (kp + 1) + 8 * kp) + sizeof(double) * static_cast<size_t>(2 * kp);
   ensure_dynamic_smem(reinterpret_cast<const void*>(chol_rinv_blocked_kernel<T, CPLX>), smem);
   // shifted CholeskyQR (Fukaya et al., SIAM J. Sci. Comput. 42 (2020) A477):
   // s = 11 (m n + n (n+1)) u ||X||_2^2 with ||X||_2^2 <= k for unit columns
   const double u = 1.1102230246251565e-16;
   const double s = shift ? 11.0 * (static_cast<double>(n) * k + static_cast<double>(k) * (k + 1)) * u * k : 0.0;
   ProfScope ps(PK_SOLVER, st, (CPLX ? 4.0 : 1.0) * 2.0 * static_cast<double>(k) * k * k / 3.0, 0.0);
-  chol_rinv_blocked_kernel<T, CPLX><<<1, 512, smem, st>>>(parts, nparts, static_cast<int>(k), s, Rinv, flag);
+  chol_rinv_blocked_kernel<T, CPLX><<<1, 512, smem, st>>>(gram, static_cast<int>(k), s, Rinv, flag);
   TG_CHECK_LAUNCH();
   count_launch();
 }
@@ -2910,7 +2922,7 @@ void chol_rinv(const T* parts, int nparts, int64_t k, int64_t n, int shift, T* R
 #define TG_INST(T)                                                                               \
   template void sum_partials<T>(const T*, int, int64_t, T*, cudaStream_t);                       \
   template void add_noise<T>(T*, int64_t, double, uint64_t, cudaStream_t);                    \
-  template void chol_rinv<T>(const T*, int, int64_t, int64_t, int, T*, int*, cudaStream_t);        \
+  template void chol_rinv<T>(const T*, int64_t, int64_t, int, T*, int*, cudaStream_t);        \
   template void counter_normal<T>(T*, int64_t, int64_t, uint64_t, uint64_t, cudaStream_t);       \
   template void upper_to_rh<T>(const T*, int64_t, int64_t, T*, cudaStream_t);                    \
   template void gemm<T>(const T*, const T*, T*, const GemmDesc&, cudaStream_t);                  \

@@ -100,7 +100,10 @@ struct EngineT final : Engine {
   static constexpr int kInfoSlots = 4096;
   int* d_info = nullptr;  // one slot per cuSOLVER call, checked at sync points
   int info_used = 0;
-  int* d_flag = nullptr;  // one per stream slot: set by device kernels on a numerical failure
+  // one per stream slot, set by device kernels on a numerical failure; then the
+  // simple update's and the dense SVD's (d_su_flag, d_svd_flag)
+  static constexpr int kFlags = kRowStreams + 3;
+  int* d_flag = nullptr;
   uint64_t noise_stream = 0;  // key sequence of the orthonormalisation perturbations
   int* d_cut = nullptr;
   // Simple-update weights on the device, [(site * 4 + leg) * lam_ld + j]: the
@@ -110,6 +113,7 @@ struct EngineT final : Engine {
   int lam_ld = 1;
   bool lam_dev_stale = true, lam_host_stale = false;
   int* d_su_flag = nullptr;
+  int* d_svd_flag = nullptr;
   std::map<std::vector<double>, DT<T>> op_cache;  // evolution operators already on the device
   const T** d_ptrs = nullptr;
   const T** h_ptrs = nullptr;  // pinned
@@ -161,14 +165,14 @@ struct EngineT final : Engine {
     TG_CUDA(cudaMalloc(&d_max, sizeof(unsigned long long) * (kRowStreams + 1)));
     TG_CUDA(cudaMalloc(&d_info, sizeof(int) * kInfoSlots));
     TG_CUDA(cudaMemset(d_info, 0, sizeof(int) * kInfoSlots));
-    TG_CUDA(cudaMalloc(&d_flag, sizeof(int) * (kRowStreams + 1)));
-    TG_CUDA(cudaMemset(d_flag, 0, sizeof(int) * (kRowStreams + 1)));
+    TG_CUDA(cudaMalloc(&d_flag, sizeof(int) * kFlags));
+    TG_CUDA(cudaMemset(d_flag, 0, sizeof(int) * kFlags));
+    d_su_flag = d_flag + kRowStreams + 1;
+    d_svd_flag = d_flag + kRowStreams + 2;
     TG_CUDA(cudaMalloc(&d_cut, sizeof(int) * (kRowStreams + 1)));
     for (int i = 0; i < lat.N; ++i)
       for (int l = 0; l < 4; ++l) lam_ld = std::max(lam_ld, lat.vdim[i][l]);
     TG_CUDA(cudaMalloc(&d_lam, sizeof(double) * 4 * lat.N * lam_ld));
-    TG_CUDA(cudaMalloc(&d_su_flag, sizeof(int)));
-    TG_CUDA(cudaMemset(d_su_flag, 0, sizeof(int)));
     TG_CUDA(cudaMalloc(&d_ptrs, sizeof(T*) * 4 * lat.N));
     TG_CUDA(cudaMallocHost(&h_ptrs, sizeof(T*) * 4 * lat.N));
     TG_CUDA(cudaMallocHost(&h_sig, sizeof(double) * 4 * lat.N));
@@ -234,7 +238,6 @@ struct EngineT final : Engine {
     cudaFree(d_flag);
     cudaFree(d_cut);
     cudaFree(d_lam);
-    cudaFree(d_su_flag);
     cudaFree(d_ptrs);
     cudaFreeHost(h_ptrs);
     cudaFreeHost(h_sig);
@@ -517,20 +520,17 @@ struct EngineT final : Engine {
   // Every cuSOLVER call reports into its own device slot; a non-zero value
   // (illegal argument or non-convergence) is turned into an error here.
   void check_infos() {
-    int flags[kRowStreams + 1] = {};
+    int flags[kFlags] = {};
     TG_CUDA(cudaMemcpyAsync(flags, d_flag, sizeof(flags), cudaMemcpyDeviceToHost, st));
     TG_CUDA(cudaStreamSynchronize(st));
     int flag = 0;
     for (int f : flags) flag |= f;
     if (flag) {
       TG_CUDA(cudaMemsetAsync(d_flag, 0, sizeof(flags), st));
+      if (flags[kRowStreams + 1])
+        fail(TG_E_RUNTIME, "simple update: the SVD of Theta did not converge (bond left unchanged)");
+      if (flags[kRowStreams + 2]) fail(TG_E_RUNTIME, "a projector matrix holds a value that is not finite");
       fail(TG_E_RUNTIME, "CholeskyQR orthonormalisation met a non-positive pivot (rank-deficient panel)");
-    }
-    TG_CUDA(cudaMemcpyAsync(&flag, d_su_flag, sizeof(int), cudaMemcpyDeviceToHost, st));
-    TG_CUDA(cudaStreamSynchronize(st));
-    if (flag) {
-      TG_CUDA(cudaMemsetAsync(d_su_flag, 0, sizeof(int), st));
-      fail(TG_E_RUNTIME, "simple update: the SVD of Theta did not converge (bond left unchanged)");
     }
     if (P.mixed && tc_fault_take())
       fail(TG_E_RUNTIME, "tensor-core product stopped waiting for its MMAs (results discarded)");
@@ -1080,9 +1080,13 @@ struct EngineT final : Engine {
   // the projectors of a line with a D = 1 leg are that narrow).  Outputs as
   // svd(): U (nrow x k), s (k, descending), VT (k x ncol), row-major.
   // Returns false (computing nothing) for other shapes, which keep gesvd.
-  bool small_side_svd(const DT<T>& Min, int64_t nrow, int64_t ncol, DT<T>& U, DT<double>& s, DT<T>& VT) {
+  static bool small_side(int64_t nrow, int64_t ncol) {
     const int64_t k = std::min(nrow, ncol);
-    if (k < 2 || k > jacobi_svd_max_k<T>() || std::max(nrow, ncol) < 4 * k) return false;
+    return k >= 2 && k <= jacobi_svd_max_k<T>() && std::max(nrow, ncol) >= 4 * k;
+  }
+  bool small_side_svd(const DT<T>& Min, int64_t nrow, int64_t ncol, DT<T>& U, DT<double>& s, DT<T>& VT) {
+    if (!small_side(nrow, ncol)) return false;
+    const int64_t k = std::min(nrow, ncol);
     const DT<T> M = reshape(Min, {nrow, ncol});
     PrecScope fp64(this, 0);  // every product of the factorisation in FP64
     DT<T> Ub({k, k}, st), Wb({k, k}, st);
@@ -1120,7 +1124,7 @@ struct EngineT final : Engine {
         U = DT<T>({nrow, k}, st);
         s = DT<double>({k}, st);
         VT = DT<T>({k, ncol}, st);
-        dense_svd<T>(M.p, nrow, ncol, U.p, s.p, VT.p, info_slot(), st);
+        dense_svd<T>(M.p, nrow, ncol, U.p, s.p, VT.p, d_svd_flag, st);
       } else {
         svd(M, nrow, ncol, U, s, VT);
       }
@@ -1776,17 +1780,24 @@ struct EngineT final : Engine {
 
   // ------------------------------------------------ CUDA-graph sweep
   //
-  // With rSVD corner projectors a sweep has no host synchronisation and all
-  // shapes are static (the environment is kept at chi), so one sweep is
+  // Where no projector waits for the host (sweep_on_device) a sweep has no host
+  // synchronisation and all shapes are static (the environment is kept at chi), so one sweep is
   // captured into a CUDA graph and replayed: ~4000 launches become one
   // graph launch.  The graph bakes in the addresses of the site tensors,
   // their rotations and the environment; it is re-captured when any of them
   // changes.  The first sweep after a change runs eagerly (it also fixes the
-  // kernels' shared-memory attributes), the second is captured.
+  // kernels' shared-memory attributes), the second is captured -- unless the
+  // caller's limit on sweeps is too near for that to pay: capturing and
+  // instantiating costs what five replays (2 x 1, D = 3, chi = 15: 13 ms, and 2.7
+  // ms gained a replay) to ten (4 x 4, chi = 48: 45 and 4.3 ms) gain, so with fewer
+  // than kCaptureSweeps sweeps to come they run eagerly until that many have.
+  static constexpr int kCaptureSweeps = 6;
   cudaGraphExec_t g_exec = nullptr;
   std::vector<const void*> g_addr;
   uint64_t g_kernels = 0;
-  bool g_warm = false, g_broken = false;
+  int g_infos = 0;  // cuSOLVER status slots that a replay writes
+  int g_eager = 0;  // sweeps run eagerly since the last change
+  bool g_broken = false;
 
   std::vector<const void*> state_addresses() {
     std::vector<const void*> a;
@@ -1804,10 +1815,34 @@ struct EngineT final : Engine {
   }
 
   bool graph_capable() const {
-    if (!P.cuda_graph || g_broken || !P.use_rsvd || !P.projector_corner || profile_enabled()) return false;
+    return P.cuda_graph && !g_broken && !profile_enabled() && sweep_on_device();
+  }
+  // Whether no projector of a sweep waits for the host: identity and randomised
+  // projectors, and the full-SVD ones that neither an ExactSolve (residuals read
+  // back) nor gesvd (host iterations) computes.
+  bool sweep_on_device() const {
     for (int i = 0; i < lat.N; ++i)
-      for (int l = 0; l < 4; ++l)
-        if (lat.vdim[i][l] == 1) return false;  // D = 1 legs can select the full-SVD branch
+      for (int r = 0; r < 4; ++r) {  // row i of the left move, in the lattice turned r times
+        const auto neighbour = [&](int site, int way) {
+          switch ((way + r) % 4) {
+            case 0: return lat.left(site);
+            case 1: return lat.top(site);
+            case 2: return lat.right(site);
+            default: return lat.bottom(site);
+          }
+        };
+        const auto leg = [&](int site, int way) { return static_cast<int64_t>(lat.vdim[site][(way + r) % 4]); };
+        if (leg(i, 3) == 1) continue;
+        if (!P.projector_corner) {
+          if (!P.use_rsvd || leg(neighbour(i, 2), 3) == 1) return false;
+          continue;
+        }
+        const int64_t t12 = leg(i, 2), t34 = leg(neighbour(i, 3), 2);
+        if (P.use_rsvd && t12 != 1 && t34 != 1) continue;
+        const int64_t nrow = t12 * P.chi * (density ? 1 : t12), ncol = t34 * P.chi * (density ? 1 : t34);
+        if (P.svd_solver != 0 || exact_block(std::min(nrow, ncol)) > 0) return false;
+        if (!small_side(nrow, ncol) && (last_bits() || !dense_svd_supported<T>(nrow, ncol))) return false;
+      }
     return true;
   }
 
@@ -1815,11 +1850,12 @@ struct EngineT final : Engine {
     if (g_exec) cudaGraphExecDestroy(g_exec);
     g_exec = nullptr;
     g_addr.clear();
-    g_warm = false;
+    g_eager = 0;
   }
 
   void capture_sweep() {
     drop_graph();
+    check_infos();  // the captured calls take their status slots from the first one on
     const uint64_t before = launch_count();
     TG_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
     cudaGraph_t g = nullptr;
@@ -1830,11 +1866,14 @@ struct EngineT final : Engine {
       if (g) cudaGraphDestroy(g);
       cudaGetLastError();
       g_broken = true;  // eager sweeps from now on
+      info_used = 0;
       uncount_launch(launch_count() - before);
       return;
     }
     TG_CUDA(cudaStreamEndCapture(st, &g));
     g_kernels = launch_count() - before;
+    g_infos = info_used;
+    info_used = 0;
     uncount_launch(g_kernels);  // recorded, not run
     const cudaError_t e = cudaGraphInstantiate(&g_exec, g, 0);
     cudaGraphDestroy(g);
@@ -1847,7 +1886,8 @@ struct EngineT final : Engine {
     g_addr = state_addresses();
   }
 
-  void run_sweep() {
+  // `left`: sweeps that may still come, this one included
+  void run_sweep(int left) {
     if (!graph_capable()) {
       sweep_impl();
       return;
@@ -1855,9 +1895,9 @@ struct EngineT final : Engine {
     const std::vector<const void*> addr = state_addresses();  // also refreshes the rotations
     if (!g_exec || addr != g_addr) {
       if (g_exec) drop_graph();
-      if (!g_warm) {
+      if (g_eager < (left >= kCaptureSweeps ? 1 : kCaptureSweeps)) {
         sweep_impl();
-        g_warm = true;
+        ++g_eager;
         return;
       }
       capture_sweep();
@@ -1866,13 +1906,15 @@ struct EngineT final : Engine {
         return;
       }
     }
+    if (g_infos > 0) check_infos();  // the slots the replay is about to write
     TG_CUDA(cudaGraphLaunch(g_exec, st));
+    info_used = g_infos;
     count_launch(g_kernels);
   }
 
   void ctm_sweep() override {
     require_env();
-    run_sweep();
+    run_sweep(kCaptureSweeps);  // no limit is known
     check_infos();
     TG_CUDA(cudaStreamSynchronize(st));
   }
@@ -1927,7 +1969,7 @@ struct EngineT final : Engine {
     int count = 0, conv = 0;
     double smax = 0.0;
     while (!conv && count < P.max_ctm_iteration) {
-      run_sweep();
+      run_sweep(P.max_ctm_iteration - count);
       check_convergence(&conv, &smax);
       ++count;
     }

@@ -402,6 +402,8 @@ tg_status tg_svd_host(int64_t m, int64_t n, int is_complex, const double* A, dou
  * pivot was not positive.  k <= 96.  For tests of the kernel; the CTMRG path
  * calls it inside the rSVD projectors (src/iTPS/core/ctm.cpp:243-244). */
 tg_status tg_cholqr_host(int64_t n, int64_t k, double* Y, int passes, int* pivot_flag);
+// The same for a complex panel (interleaved real and imaginary parts, k <= 88).
+tg_status tg_cholqr_host_complex(int64_t n, int64_t k, double* Y, int passes, int* pivot_flag);
 
 /* Allocation-free corner spectra.  No counterpart in the reference: it exists
  * for callers that must not allocate device memory where they need the

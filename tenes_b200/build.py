@@ -20,7 +20,7 @@ ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 BUILD = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libtenes_gpu.so")
-SOURCES = ["kernels.cu", "cholqr.cu", "skinny.cu", "tile_gemm.cu", "jacobi.cu", "dense_svd.cu", "su_fused.cu", "adjoint.cu", "engine.cu", "api.cu",
+SOURCES = ["kernels.cu", "cholqr.cu", "cholqr_complex.cu", "skinny.cu", "tile_gemm.cu", "jacobi.cu", "dense_svd.cu", "su_fused.cu", "adjoint.cu", "engine.cu", "api.cu",
            "noalloc.cu", "main_entry.cpp"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 

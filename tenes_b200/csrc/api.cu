@@ -503,22 +503,27 @@ extern "C" tg_status tg_gemm_group_stats(int64_t* tuned, int64_t* wins, int nwin
   return guard([&] { tg::gemm_group_stats(tuned, wins, nwins); });
 }
 
-extern "C" tg_status tg_cholqr_host(int64_t n, int64_t k, double* Y, int passes, int* pivot_flag) {
+static tg_status cholqr_host(int64_t n, int64_t k, double* Y, int passes, int* pivot_flag, bool complex) {
   return guard([&] {
     if (n < 1 || k < 1 || k > n || passes < 1 || !Y) tg::fail(TG_E_INPUT, "bad CholeskyQR arguments");
-    if (!tg::cholqr_cluster_supported(n, k)) tg::fail(TG_E_INPUT, "CholeskyQR panel shape not supported");
+    if (!(complex ? tg::cholqr_complex_supported(n, k) : tg::cholqr_cluster_supported(n, k)))
+      tg::fail(TG_E_INPUT, "CholeskyQR panel shape not supported");
+    const size_t bytes = sizeof(double) * n * k * (complex ? 2 : 1);
+    const double noise = 1e-14 / std::sqrt(static_cast<double>(n));
     cudaStream_t st;
     TG_CUDA(cudaStreamCreate(&st));
     double *dY = nullptr, *dscr = nullptr;
     int* dflag = nullptr;
-    TG_CUDA(cudaMalloc(&dY, sizeof(double) * n * k));
-    TG_CUDA(cudaMalloc(&dscr, sizeof(double) * tg::cholqr_scratch_doubles(k)));
+    TG_CUDA(cudaMalloc(&dY, bytes));
+    TG_CUDA(cudaMalloc(&dscr, sizeof(double) * (complex ? tg::cholqr_complex_scratch_doubles(k)
+                                                        : tg::cholqr_scratch_doubles(k))));
     TG_CUDA(cudaMalloc(&dflag, sizeof(int)));
     TG_CUDA(cudaMemsetAsync(dflag, 0, sizeof(int), st));
-    TG_CUDA(cudaMemcpyAsync(dY, Y, sizeof(double) * n * k, cudaMemcpyHostToDevice, st));
-    tg::cholqr_cluster(dY, n, k, passes, 2, 1, 1e-14 / std::sqrt(static_cast<double>(n)), dscr, dflag, st);
+    TG_CUDA(cudaMemcpyAsync(dY, Y, bytes, cudaMemcpyHostToDevice, st));
+    if (complex) tg::cholqr_complex(reinterpret_cast<tg::cplx*>(dY), n, k, passes, 2, 1, noise, dscr, dflag, st);
+    else tg::cholqr_cluster(dY, n, k, passes, 2, 1, noise, dscr, dflag, st);
     int flag = 0;
-    TG_CUDA(cudaMemcpyAsync(Y, dY, sizeof(double) * n * k, cudaMemcpyDeviceToHost, st));
+    TG_CUDA(cudaMemcpyAsync(Y, dY, bytes, cudaMemcpyDeviceToHost, st));
     TG_CUDA(cudaMemcpyAsync(&flag, dflag, sizeof(int), cudaMemcpyDeviceToHost, st));
     TG_CUDA(cudaStreamSynchronize(st));
     cudaFree(dY);
@@ -527,6 +532,14 @@ extern "C" tg_status tg_cholqr_host(int64_t n, int64_t k, double* Y, int passes,
     cudaStreamDestroy(st);
     if (pivot_flag) *pivot_flag = flag;
   });
+}
+
+extern "C" tg_status tg_cholqr_host(int64_t n, int64_t k, double* Y, int passes, int* pivot_flag) {
+  return cholqr_host(n, k, Y, passes, pivot_flag, false);
+}
+
+extern "C" tg_status tg_cholqr_host_complex(int64_t n, int64_t k, double* Y, int passes, int* pivot_flag) {
+  return cholqr_host(n, k, Y, passes, pivot_flag, true);
 }
 
 extern "C" tg_status tg_bench_gemm(int64_t M, int64_t N, int64_t K, int layout, int prec, int iters,

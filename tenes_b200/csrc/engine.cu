@@ -778,12 +778,22 @@ struct EngineT final : Engine {
   // iteration, whose next product and orthonormalisation only use the span.
   // (One shifted pass is not enough: with weakly converged site tensors the
   // next panel's Gram matrix then met a non-positive pivot.)
-  void orth_chol(DT<T>& Y, int64_t n, int64_t k, int passes = 4) {
+  //
+  // free_order: the caller's results do not hang on the roundings of the complex
+  // panels' Gram / factor / product launches, which one cluster launch replaces.
+  void orth_chol(DT<T>& Y, int64_t n, int64_t k, int passes = 4, bool free_order = false) {
     PrecScope fp64(this, 0);
     if constexpr (!CPLX) {
       if (cholqr_cluster_supported(n, k)) {
         DT<double> scratch({cholqr_scratch_doubles(k)}, st);
         cholqr_cluster(Y.p, n, k, passes, 2, ++noise_stream, 1e-14 / std::sqrt(static_cast<double>(n)), scratch.p,
+                       d_flag + slot, st);
+        return;
+      }
+    } else {
+      if (free_order && cholqr_complex_supported(n, k)) {
+        DT<double> scratch({cholqr_complex_scratch_doubles(k)}, st);
+        cholqr_complex(Y.p, n, k, passes, 2, ++noise_stream, 1e-14 / std::sqrt(static_cast<double>(n)), scratch.p,
                        d_flag + slot, st);
         return;
       }
@@ -954,7 +964,7 @@ struct EngineT final : Engine {
     }
     void orth(DT<T>& X, int64_t n, int passes) {
       if (householder) e->orth_cm(X, n, b);
-      else e->orth_chol(X, n, b, passes);
+      else e->orth_chol(X, n, b, passes, !e->keep_order());
     }
     void start() {
       PrecScope fp64(e, 0);

@@ -239,6 +239,14 @@ int64_t cholqr_scratch_doubles(int64_t k);
 void cholqr_cluster(double* Y, int64_t n, int64_t k, int passes, int shifted_passes, uint64_t noise_stream,
                     double noise_scale, double* scratch, int* flag, cudaStream_t st);
 
+// The same for a complex panel, k <= 88, in scratch of
+// cholqr_complex_scratch_doubles(k) doubles.  (chol_rinv's form rounds
+// differently: the randomised projectors keep that one.)
+bool cholqr_complex_supported(int64_t n, int64_t k);
+int64_t cholqr_complex_scratch_doubles(int64_t k);
+void cholqr_complex(cplx* Y, int64_t n, int64_t k, int passes, int shifted_passes, uint64_t noise_stream,
+                    double noise_scale, double* scratch, int* flag, cudaStream_t st);
+
 // y += alpha x (alpha real)
 template <typename T>
 void axpy(T* y, const T* x, double alpha, int64_t n, cudaStream_t st);

@@ -1801,6 +1801,10 @@ struct EngineT final : Engine {
   // instantiating costs what five replays (2 x 1, D = 3, chi = 15: 13 ms, and 2.7
   // ms gained a replay) to ten (4 x 4, chi = 48: 45 and 4.3 ms) gain, so with fewer
   // than kCaptureSweeps sweeps to come they run eagerly until that many have.
+  // Randomised corner projectors alone are captured at the second sweep whatever
+  // the limit: it shortens every run after the first by more (3 x 2, D = 3, chi =
+  // 11, two sweeps a run: 36.5, then 15.8 ms a run, against three of 21.1 and one
+  // of 33.4 before the first of 15.8).
   static constexpr int kCaptureSweeps = 6;
   cudaGraphExec_t g_exec = nullptr;
   std::vector<const void*> g_addr;
@@ -1824,6 +1828,13 @@ struct EngineT final : Engine {
     return a;
   }
 
+  bool randomised_corners() const {
+    if (!P.projector_corner || !P.use_rsvd) return false;
+    for (const auto& legs : lat.vdim)
+      for (int leg = 0; leg < 4; ++leg)
+        if (legs[leg] == 1) return false;
+    return true;
+  }
   bool graph_capable() const {
     return P.cuda_graph && !g_broken && !profile_enabled() && sweep_on_device();
   }
@@ -1905,7 +1916,7 @@ struct EngineT final : Engine {
     const std::vector<const void*> addr = state_addresses();  // also refreshes the rotations
     if (!g_exec || addr != g_addr) {
       if (g_exec) drop_graph();
-      if (g_eager < (left >= kCaptureSweeps ? 1 : kCaptureSweeps)) {
+      if (g_eager < (left >= kCaptureSweeps || randomised_corners() ? 1 : kCaptureSweeps)) {
         sweep_impl();
         ++g_eager;
         return;

@@ -4,7 +4,9 @@
 // (same tensordot sequences, same leg orders), so every intermediate can be
 // compared one to one with the reference algorithm.  All tensors stay on the
 // device; contractions run on the hand-written DMMA kernels of kernels.cu,
-// the dense projector SVD and the simple-update QR / SVD on cuSOLVER.
+// tile_gemm.cu and skinny.cu, the projectors' factorisations on cholqr.cu,
+// cholqr_complex.cu, jacobi.cu and dense_svd.cu, the bond steps on su_fused.cu;
+// what those do not take is left to cuSOLVER.
 #include <cusolverDn.h>
 
 #include <algorithm>

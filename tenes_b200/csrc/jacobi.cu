@@ -34,6 +34,7 @@
 
 #include "kernels.cuh"
 #include "rotation.cuh"
+#include "scaling.cuh"
 
 namespace tg {
 namespace {
@@ -206,7 +207,9 @@ __device__ double block_sum(double a) {
 // kSvd, kCircle: column norms descending to S, the normalised columns in that
 // order to U, the rotations to `log` (round-major) and {sweeps, position of
 // every column} to `info`.  kSpectrum: the norms, divided by their 2-norm,
-// descending to S, one matrix a CTA (mats[blockIdx.x]).
+// descending to S, one matrix a CTA (mats[blockIdx.x]).  Both of kSvd and
+// kSpectrum scale a matrix far from 1 by a power of two first: the rotation
+// test squares the columns' inner products, the fourth power of the entries.
 // WIDE: more columns than the CTA's lanes can hold; a group takes several pairs
 // of a circle tournament in turn.
 enum JacobiMode { kSpectrum, kSvd, kCircle };
@@ -231,9 +234,11 @@ __global__ void __launch_bounds__(THREADS)
   const int g = tid / LANES, gl = tid % LANES;
 
   double total = 0.0;
+  int top = 0;
   for (int idx = tid; idx < nn; idx += blockDim.x) {
     const int r = idx / n, c = idx % n;
     const T v = A[idx];
+    if constexpr (MODE != kCircle) top = max(top, magnitude(v));
     ar[c * LD + r] = re_of(v);
     total = fma(re_of(v), re_of(v), total);
     if constexpr (CPLX) {
@@ -246,7 +251,24 @@ __global__ void __launch_bounds__(THREADS)
     ar[c * LD + r] = 0.0;
     if constexpr (CPLX) ai[c * LD + r] = 0.0;
   }
+  __shared__ int warp_top[32];
+  if constexpr (MODE != kCircle) {
+    top = __reduce_max_sync(0xffffffffu, top);
+    if (lane == 0) warp_top[warp] = top;
+  }
   total = block_sum(total);  // its barriers also order the stores above
+  double unscale = 1.0;
+  if constexpr (MODE != kCircle) {
+    const double scale = range_scale(__reduce_max_sync(0xffffffffu, lane < nw ? warp_top[lane] : 0), unscale);
+    if (scale != 1.0) {  // the same in every thread
+      total = 0.0;
+      for (int idx = tid; idx < (CPLX ? 2 : 1) * n * LD; idx += blockDim.x) {  // both planes
+        ar[idx] *= scale;
+        total = fma(ar[idx], ar[idx], total);
+      }
+      total = block_sum(total);
+    }
+  }
   const double tol = static_cast<double>(n) * 2.220446049250313e-16, tol2 = tol * tol;
   const double small2 = tol2 * total;  // columns of rounding noise
 
@@ -431,7 +453,7 @@ __global__ void __launch_bounds__(THREADS)
       const double w = nrm[o];
       pos += (w > v) || (w == v && o < c);
     }
-    S[pos] = VEC ? v : (unit > 0.0 ? v / unit : 0.0);
+    S[pos] = VEC ? v * unscale : (unit > 0.0 ? v / unit : 0.0);
     if (VEC) info[1 + c] = pos;
   }
   if constexpr (VEC) {

@@ -11,12 +11,17 @@
 #include <cstdint>
 
 #include "kernels.cuh"
+#include "scaling.cuh"
 
 namespace tg {
 namespace {
 
 constexpr int kQrThreads = 512;
 constexpr size_t kSmemMax = 227 * 1024;
+// a column of a smaller norm (squared) is lifted before its reflector is made:
+// its squares lose digits, and the reflector would not be unitary
+constexpr double kTinyNorm2 = 1e-240;
+constexpr double kLift = 3.273390607896142e150, kUnlift = 3.054936363499605e-151;  // 2^500, 2^-500
 
 __device__ __forceinline__ double conj_of(double x) { return x; }
 __device__ __forceinline__ cplx conj_of(cplx x) { return make_double2(x.x, -x.y); }
@@ -27,6 +32,8 @@ __device__ __forceinline__ double real_of(cplx x) { return x.x; }
 __device__ __forceinline__ double imag_of(double) { return 0.0; }
 __device__ __forceinline__ double imag_of(cplx x) { return x.y; }
 __device__ __forceinline__ double mul(double a, double b) { return a * b; }
+__device__ __forceinline__ double times(double a, double b) { return a * b; }
+__device__ __forceinline__ cplx times(cplx a, double b) { return make_double2(a.x * b, a.y * b); }
 __device__ __forceinline__ cplx mul(cplx a, cplx b) {
   return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
@@ -54,7 +61,8 @@ __device__ __forceinline__ cplx warp_sum(cplx v) { return make_double2(warp_sum(
 // column of A at place c.  One CTA, the matrix in shared memory; every warp
 // holds the reflector of a step in registers (computed by each warp for itself,
 // so a step has one barrier) and applies it to its share of the columns.
-// *info is set to 1 when the matrix holds a value that is not finite.
+// *info is set to 1 when the matrix holds a value that is not finite.  A matrix
+// far from unit scale is factored times a power of two, which L takes out again.
 template <typename T, int RPL>
 __global__ void __launch_bounds__(kQrThreads)
     sorted_qr_kernel(const T* __restrict__ M, int64_t sr, int64_t sc, bool conj, int m, int k, T* __restrict__ V,
@@ -65,12 +73,26 @@ __global__ void __launch_bounds__(kQrThreads)
   double* nrm = reinterpret_cast<double*>(a + static_cast<size_t>(ld) * k);
   int* at = reinterpret_cast<int*>(nrm + k);                 // place c holds column at[c]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
+  __shared__ int warp_top[kQrThreads / 32];
+  int top = 0;
   for (int idx = tid; idx < m * k; idx += blockDim.x) {
     const int r = sc == 1 ? idx / k : idx % m, c = sc == 1 ? idx % k : idx / m;
     const T v = M[r * sr + c * sc];
+    top = max(top, magnitude(v));
     a[c * ld + r] = conj ? conj_of(v) : v;
   }
+  top = __reduce_max_sync(0xffffffffu, top);
+  if (lane == 0) warp_top[warp] = top;
   __syncthreads();
+  top = __reduce_max_sync(0xffffffffu, lane < nw ? warp_top[lane] : 0);
+  double unscale;
+  const double range = range_scale(top, unscale);
+  if (range != 1.0) {  // the same in every thread
+    for (int idx = tid; idx < ld * k; idx += blockDim.x)
+      if (idx % ld < m) a[idx] = times(a[idx], range);
+    __syncthreads();
+  }
+  if (tid == 0 && top >= 0x7ff00000 && info) atomicExch(info, 1);
   for (int c = warp; c < k; c += nw) {
     double s = 0.0;
     for (int r = lane; r < m; r += 32) s += abs2(a[c * ld + r]);
@@ -78,7 +100,6 @@ __global__ void __launch_bounds__(kQrThreads)
     if (lane == 0) {
       nrm[c] = s;
       at[c] = c;
-      if (!(s <= 1.7976931348623157e308) && info) atomicExch(info, 1);
     }
   }
   __syncthreads();
@@ -101,7 +122,29 @@ __global__ void __launch_bounds__(kQrThreads)
       s += abs2(v[i]);
     }
     s = warp_sum(s);
-    const T alpha = x[j];
+    T alpha = x[j];
+    double unlift = unscale;
+    if (fma(real_of(alpha), real_of(alpha), fma(imag_of(alpha), imag_of(alpha), s)) < kTinyNorm2) {
+      bool some = imag_of(alpha) != 0.0;
+#pragma unroll
+      for (int i = 0; i < RPL; ++i) some = some || magnitude(v[i]) != 0;
+      if (__any_sync(0xffffffffu, some)) {  // not for the zero columns of a padded matrix
+        s = 0.0;
+#pragma unroll
+        for (int i = 0; i < RPL; ++i) {
+          v[i] = times(v[i], kLift);
+          s += abs2(v[i]);
+        }
+        s = warp_sum(s);
+        alpha = times(alpha, kLift);
+        unlift *= kUnlift;
+        if (fma(real_of(alpha), real_of(alpha), fma(imag_of(alpha), imag_of(alpha), s)) < kTinyNorm2) {
+          // nothing against the matrix, 1e-240 of it: no reflector
+          s = 0.0;
+          alpha = make<T>(real_of(alpha), 0.0);
+        }
+      }
+    }
     const double ar = real_of(alpha), ai = imag_of(alpha);
     double beta = ar;
     T t = make<T>(0.0, 0.0);
@@ -127,7 +170,7 @@ __global__ void __launch_bounds__(kQrThreads)
     }
     // L = R^H: row c, column j <= c holds conj(R(j, c))
     if (tid < j) L[static_cast<int64_t>(tid) * k + j] = make<T>(0.0, 0.0);
-    if (tid == j) L[static_cast<int64_t>(j) * k + j] = make<T>(beta, 0.0);
+    if (tid == j) L[static_cast<int64_t>(j) * k + j] = make<T>(beta * unlift, 0.0);
     const T tc = conj_of(t);
     for (int c = j + 1 + warp; c < k; c += nw) {
       T* y = a + at[c] * ld;
@@ -145,7 +188,7 @@ __global__ void __launch_bounds__(kQrThreads)
         if (r >= j && r < m) {
           const T u = sub(z[i], mul(v[i], d));
           y[r] = u;
-          if (r == j) L[static_cast<int64_t>(c) * k + j] = conj_of(u);
+          if (r == j) L[static_cast<int64_t>(c) * k + j] = times(conj_of(u), unscale);
         }
       }
     }

@@ -44,3 +44,35 @@ def test_corner_spectrum(chi, is_complex):
         # normalised by its 2-norm; 32 n u as above
         assert np.abs(env.corner_spectrum(0, 0) - ref / np.linalg.norm(ref)).max() <= 32 * chi * U
     env.close()
+
+
+def dense_svd(A):
+    m, n = A.shape
+    k = min(m, n)
+    Uo, VT, S = np.empty((m, k), A.dtype), np.empty((k, n), A.dtype), np.empty(k)
+    check(_lib.load().tg_svd_host(m, n, int(np.iscomplexobj(A)), dptr(A), dptr(Uo), dptr(S), dptr(VT)))
+    return Uo, S, VT
+
+
+@pytest.mark.parametrize("is_complex", [False, True])
+@pytest.mark.parametrize("m,n", [(12, 12), (33, 20), (40, 90)])
+def test_dense_svd(m, n, is_complex):
+    A = matrix(max(m, n), is_complex, m + n)[:m, :n]
+    tol = 40 * min(m, n) * U * np.linalg.norm(A)  # the bound at unit scale (test_gpu_dense_svd.py)
+    for scale in SCALES + [1e160, 1e300]:
+        Uo, S, VT = dense_svd(np.ascontiguousarray(A * scale))
+        assert np.abs(S / scale - np.linalg.svd(A, compute_uv=False)).max() <= tol
+        assert np.linalg.norm(Uo * (S / scale) @ VT - A) <= tol
+
+
+@pytest.mark.parametrize("is_complex", [False, True])
+@pytest.mark.parametrize("tiny", [1e-110, 1e-158, 1e-170, 1e-260, 1e-300])
+def test_dense_svd_tiny_columns(tiny, is_complex):
+    """Columns whose squares lose digits or vanish beside ordinary ones."""
+    m, n, live = 24, 20, 14
+    A = np.ascontiguousarray(matrix(m, is_complex, 3)[:, :n] * np.where(np.arange(n) < live, 1.0, tiny))
+    Uo, S, VT = dense_svd(A)
+    tol = 40 * n * U
+    assert np.linalg.norm(Uo * S @ VT - A) <= tol * np.linalg.norm(A)
+    assert np.abs(Uo[:, :live].conj().T @ Uo[:, :live] - np.eye(live)).max() <= tol
+    assert np.abs(VT[:live] @ VT[:live].conj().T - np.eye(live)).max() <= tol

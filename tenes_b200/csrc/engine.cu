@@ -26,6 +26,7 @@
 #include "local_gauge.hpp"
 #include "dtensor.hpp"
 #include "engine.hpp"
+#include "exact_steps.hpp"
 #include "kernels.cuh"
 
 namespace tg {
@@ -897,7 +898,7 @@ struct EngineT final : Engine {
   // row) ended with in the previous sweep -- an almost converged guess once
   // the environment settles -- completed with counter-based Gaussian
   // columns.  If the residuals are not below the tolerance after
-  // kExactMaxIters iterations (a flat spectrum at the block edge), the
+  // ExactSteps::kMaxIters iterations (a flat spectrum at the block edge), the
   // dense SVD is used instead.
   // Contexts whose results carry the last bits of a singular vector to more
   // than nine digits: 3xTF32 products turn one into 1e-7; up/down, complex iTPO
@@ -910,11 +911,8 @@ struct EngineT final : Engine {
   bool last_bits() const { return P.mixed || !P.projector_corner || (CPLX && density); }
   bool keep_order() const { return last_bits() || narrow_bonds; }
   static constexpr double kExactTol = 1e-13;
-  static constexpr int kExactMaxIters = 80;
   std::map<int, DT<T>> warm_v;   // right basis (ncol x b, column-major) per projector
-  // iterations the same projector's last solve needed: where the next one
-  // looks first (a check costs as much as three to five iterations)
-  std::map<int, int> iter_hint;
+  std::map<int, int> iter_hint;  // where its next solve looks first (ExactSteps)
   int proj_key = -1;             // set by the moves before each projector
   int64_t exact_solves = 0, exact_iters = 0, exact_checks = 0, exact_dense = 0;
 
@@ -950,8 +948,8 @@ struct EngineT final : Engine {
     // yields orthonormal columns for any panel, before giving up for the
     // dense SVD.
     bool householder = false;
-    int it = 0, next_check = 0, prev_it = 0;
-    double prev_ratio = 0.0;
+    int it = 0, next_check = 0;
+    ExactSteps steps;
     DT<T> Q, Qz, Ur, Wr, Y;
     DT<double> s;
     DT<T> Uc, Vc;
@@ -980,11 +978,10 @@ struct EngineT final : Engine {
       }
       if (b > w0) counter_normal<T>(Om.p + static_cast<int64_t>(w0) * ncol, ncol, b - w0, e->P.rsvd_seed, 7, e->st);
       Q = e->mm_cm(m, cm(Om.p, ncol, b));  // nrow x b, column-major
-      it = prev_it = 0;
-      prev_ratio = 0.0;
+      it = 0;
+      steps = ExactSteps{e->keep_order()};
       auto last = e->iter_hint.find(key);
-      next_check = b == std::min(nrow, ncol) ? 1 : key >= 0 && last != e->iter_hint.end() ? last->second : w0 > 0 ? 2 : 3;
-      if (e->keep_order()) next_check = (w0 > 0 || b == std::min(nrow, ncol)) ? 1 : 3;
+      next_check = steps.first(w0 > 0, key >= 0 && last != e->iter_hint.end() ? last->second : 0);
       orth(Q, nrow, next_check == 1 ? 4 : 2);
       advance();
     }
@@ -1039,16 +1036,11 @@ struct EngineT final : Engine {
       double worst = 0.0;
       for (int i = 0; i < cut; ++i) worst = std::max(worst, host[b + i]);
       const double ratio = host[0] > 0.0 ? worst / (kExactTol * host[0]) : 0.0;
-      // the residual's decay an iteration: seen between the last two checks, or
-      // expected from the kept and the dropped edge of the block's spectrum
-      double decay = 0.5;
-      if (prev_it > 0 && ratio < prev_ratio) decay = std::pow(ratio / prev_ratio, 1.0 / (it - prev_it));
-      else if (cut > 0 && !e->keep_order()) decay = std::min(0.5, (host[b - 1] / host[cut - 1]) * (host[b - 1] / host[cut - 1]));
-      if (ratio <= 1.0 || b == std::min(nrow, ncol)) {
-        if (key >= 0) {  // one or two iterations fewer where the residual shows them to spare
-          int spare = 0;
-          while (spare < 2 && ratio * std::pow(decay, -(spare + 1)) <= 1.0 && decay > 0.0) ++spare;
-          e->iter_hint[key] = std::max(2, it - spare);
+      // the decay an iteration that the dropped and the kept edge of the block's spectrum promise
+      const double edge = cut > 0 ? (host[b - 1] / host[cut - 1]) * (host[b - 1] / host[cut - 1]) : 1.0;
+      if (ratio <= 1.0) {
+        if (key >= 0) {
+          e->iter_hint[key] = steps.hint(it, ratio, edge);
           if (householder) e->iter_hint.erase(key);  // a block beyond the rank: look early, to notice it again
         }
         DT<T> U = e->mm_rm(cm(Q.p, nrow, b), rm(Ur.p, b, b));   // nrow x b row-major
@@ -1062,15 +1054,8 @@ struct EngineT final : Engine {
         if (key >= 0) e->warm_v[key] = e->mm_cm(cm(Qz.p, ncol, b), rm(Wr.p, b, b));
         return kDone;
       }
-      // a stalled decay (a flat spectrum at the block edge), or too many iterations: the dense SVD
-      if (prev_it > 0 && it > 12 && ratio > 0.5 * prev_ratio) return failed();
-      // iterations to the next check
-      int gap = 3;
-      if ((prev_it == 0 ? !e->keep_order() : ratio < prev_ratio) && decay > 0.0)
-        gap = std::min(16, std::max(1, static_cast<int>(std::ceil(std::log(ratio) / -std::log(decay)))));
-      if (it + gap > kExactMaxIters) return failed();
-      prev_it = it;
-      prev_ratio = ratio;
+      const int gap = steps.next(it, ratio, edge);
+      if (gap == 0) return failed();  // a flat spectrum at the block edge: the dense SVD
       next_check = it + gap;
       Q = std::move(Y);
       orth(Q, nrow, next_check == it + 1 ? 4 : 2);

@@ -1,0 +1,73 @@
+// Where an exact truncated SVD (block subspace iteration) looks at its residuals.
+#pragma once
+
+#include <algorithm>
+#include <cmath>
+
+namespace tg {
+
+// A check (orthonormalisation, Jacobi, host read) costs three to five
+// iterations, so a solve should need one or two of them.  `ratio` is the largest
+// kept residual over the tolerance: the solve is done at ratio <= 1.
+//
+// fixed: the first check at 1 (from the basis of the last solve) or 3, the next
+// three later, the others from the decay of the last two, for contexts whose
+// results depend on where a solve ends (EngineT::keep_order).
+//
+// Otherwise the first check is where the projector's last solve in this
+// environment ended, the next ones come from the decay seen between two checks
+// or, before there are two, expected from the block's spectrum.  Against the
+// fixed places, 2 x 2 environments of D = 3 and 4, real and complex, 60 inputs:
+// 0.79 of the time, errors against 64 bits 1.3e-14 to 9.9e-14 against 1.1e-14 to
+// 8.1e-14 (geometric means of 12).
+struct ExactSteps {
+  static constexpr int kMaxIters = 80;
+
+  bool fixed = false;
+  int prev_it = 0;  // the last check, 0: none
+  double prev_ratio = 0.0;
+
+  // the first check; hint: hint() of the projector's last solve, 0: none
+  int first(bool warm, int hint) const {
+    if (fixed) return warm ? 1 : 3;
+    return hint > 0 ? hint : warm ? 2 : 3;
+  }
+  bool falling(double ratio) const { return prev_it > 0 && ratio < prev_ratio; }
+  // the residuals' decay an iteration; edge: the same expected from the spectrum
+  double decay(int it, double ratio, double edge) const {
+    return falling(ratio) ? std::pow(ratio / prev_ratio, 1.0 / (it - prev_it)) : std::min(0.5, edge);
+  }
+  // After a check at `it` with ratio > 1: iterations to the next one, or 0 for a
+  // solve to be given up (for the dense SVD).
+  int next(int it, double ratio, double edge) {
+    const double f = decay(it, ratio, edge);
+    const double need = f > 0.0 ? std::max(1.0, std::ceil(std::log(ratio) / -std::log(f))) : 3.0;
+    const int left = kMaxIters - it;
+    int gap = falling(ratio) || (prev_it == 0 && !fixed) ? static_cast<int>(std::min(16.0, need)) : 3;
+    if (fixed) {
+      if (prev_it > 0 && it > 12 && ratio > 0.5 * prev_ratio) return 0;
+    } else {
+      // stalled is what cannot end in the iterations left, by the decay of an
+      // iteration: a late first check can be followed by a gap of one, over which a
+      // sound decay is 0.8.  (Judged by a ratio of 0.5 between two checks, solves of
+      // 30 iterations at D = 4, chi = 60 went to the dense SVD.)
+      if (falling(ratio) && it > 12 && need > left) return 0;
+      if (prev_it > 0 && !falling(ratio) && it > 12 && it - prev_it >= 3) return 0;
+      if (left > 0) gap = std::min(gap, left);
+    }
+    if (gap > left) return 0;
+    prev_it = it;
+    prev_ratio = ratio;
+    return gap;
+  }
+  // After the last check, at `it`: where the next solve looks first, one or two
+  // iterations earlier where the residual shows them to spare.
+  int hint(int it, double ratio, double edge) const {
+    const double f = decay(it, ratio, edge);
+    int spare = 0;
+    while (spare < 2 && f > 0.0 && ratio * std::pow(f, -(spare + 1)) <= 1.0) ++spare;
+    return std::max(2, it - spare);
+  }
+};
+
+}  // namespace tg

@@ -897,7 +897,10 @@ struct EngineT final : Engine {
   // The start block holds the basis that the same projector (move, line,
   // row) ended with in the previous sweep -- an almost converged guess once
   // the environment settles -- completed with counter-based Gaussian
-  // columns.  If the residuals are not below the tolerance after
+  // columns.  An environment made from the site tensors, or set, starts without
+  // them (forget_solves), so that it does not depend on what the context computed
+  // before; only keep_order() contexts keep them, as their results would move
+  // with the start block.  If the residuals are not below the tolerance after
   // ExactSteps::kMaxIters iterations (a flat spectrum at the block edge), the
   // dense SVD is used instead.
   // Contexts whose results carry the last bits of a singular vector to more
@@ -915,6 +918,12 @@ struct EngineT final : Engine {
   std::map<int, int> iter_hint;  // where its next solve looks first (ExactSteps)
   int proj_key = -1;             // set by the moves before each projector
   int64_t exact_solves = 0, exact_iters = 0, exact_checks = 0, exact_dense = 0;
+
+  void forget_solves() {
+    if (keep_order()) return;
+    warm_v.clear();
+    iter_hint.clear();
+  }
 
   // block size of the subspace iteration, or -1 where the dense SVD is the
   // better choice: a matrix whose smaller dimension a block would span gains
@@ -1702,6 +1711,7 @@ struct EngineT final : Engine {
   }
 
   void ctm_init() override {
+    forget_solves();
     if (density) {
       ctm_init_density();
       return;
@@ -3357,6 +3367,7 @@ struct EngineT final : Engine {
   }
   void set_env(int which, int site, const double* host) override {
     upload(env_ref(which, site), host);  // into the existing storage (captured sweeps hold its address)
+    forget_solves();
     env_ready = true;
     spec_old_ok = false;
   }

@@ -8,14 +8,14 @@ from tenes_b200.env import CTMParams, Environment
 pytestmark = pytest.mark.gpu
 
 
-def site_tensors(dims, seed, falloff, is_complex=False):
+def site_tensors(dims, seed, falloff, is_complex=False, density=False):
     rng = np.random.default_rng(seed)
     out = []
     for d in dims:
-        shape = tuple(d) + (2,)
+        shape = tuple(d) + ((2, 2) if density else (2,))
         t = rng.normal(size=shape) + (1j * rng.normal(size=shape) if is_complex else 0)
         for leg, n in enumerate(d):
-            t = t * np.exp(-falloff * np.arange(n)).reshape([-1 if a == leg else 1 for a in range(5)])
+            t = t * np.exp(-falloff * np.arange(n)).reshape([-1 if a == leg else 1 for a in range(t.ndim)])
         out.append(t / np.abs(t).max())
     return out
 
@@ -42,3 +42,25 @@ def test_slow_decay_is_no_stall(size, is_complex):
         counts = run(env, tensors)
         assert counts["solves"] == 20 * len(dims) and counts["dense"] == 0
     env.close()
+
+
+@pytest.mark.parametrize("D,chi,is_complex,density", [(3, 24, False, False), (3, 20, True, False), (6, 24, False, True)])
+def test_from_scratch_whatever_was_before(D, chi, is_complex, density):
+    """A context that has computed another state's environment gives the same
+    environment as a new one, bit for bit, with the same iterations and checks."""
+    dims = [[D] * 4] * 4
+    first, other = (site_tensors(dims, seed, 0.4, is_complex, density) for seed in (11, 12))
+    got = []
+    for before in ([], [other], [first, other]):
+        env = Environment(2, 2, [2] * 4, dims, CTMParams(chi=chi, max_ctm_iteration=3, ctm_convergence_epsilon=1e-10,
+                                                         density=density), is_complex)
+        for tensors in before:
+            run(env, tensors)
+        counts = run(env, first)
+        assert counts["solves"] == 48
+        got.append((counts, [env.get_env(w, i) for w in range(8) for i in range(4)]))
+        env.close()
+    for counts, tensors in got[1:]:
+        assert counts == got[0][0]
+        for a, b in zip(tensors, got[0][1]):
+            assert np.array_equal(a, b)

@@ -784,20 +784,25 @@ struct EngineT final : Engine {
   //
   // free_order: the caller's results do not hang on the roundings of the complex
   // panels' Gram / factor / product launches, which one cluster launch replaces.
-  void orth_chol(DT<T>& Y, int64_t n, int64_t k, int passes = 4, bool free_order = false) {
+  // flag (device) is set on a pivot that is not positive, keys counts the
+  // perturbations; the stream slot's and the context's where null.
+  void orth_chol(DT<T>& Y, int64_t n, int64_t k, int passes = 4, bool free_order = false, int* flag = nullptr,
+                 uint64_t* keys = nullptr) {
     PrecScope fp64(this, 0);
+    if (!flag) flag = d_flag + slot;
+    if (!keys) keys = &noise_stream;
     if constexpr (!CPLX) {
       if (cholqr_cluster_supported(n, k)) {
         DT<double> scratch({cholqr_scratch_doubles(k)}, st);
-        cholqr_cluster(Y.p, n, k, passes, 2, ++noise_stream, 1e-14 / std::sqrt(static_cast<double>(n)), scratch.p,
-                       d_flag + slot, st);
+        cholqr_cluster(Y.p, n, k, passes, 2, ++*keys, 1e-14 / std::sqrt(static_cast<double>(n)), scratch.p,
+                       flag, st);
         return;
       }
     } else {
       if (free_order && cholqr_complex_supported(n, k)) {
         DT<double> scratch({cholqr_complex_scratch_doubles(k)}, st);
-        cholqr_complex(Y.p, n, k, passes, 2, ++noise_stream, 1e-14 / std::sqrt(static_cast<double>(n)), scratch.p,
-                       d_flag + slot, st);
+        cholqr_complex(Y.p, n, k, passes, 2, ++*keys, 1e-14 / std::sqrt(static_cast<double>(n)), scratch.p,
+                       flag, st);
         return;
       }
     }
@@ -807,9 +812,9 @@ struct EngineT final : Engine {
       DT<T> G({k, k}, st);
       sum_partials<T>(parts.p, nparts, k * k, G.p, st);
       DT<T> Ri({k, k}, st);
-      chol_rinv<T>(G.p, k, n, pass <= 1 ? 1 : 0, Ri.p, d_flag + slot, st);
+      chol_rinv<T>(G.p, k, n, pass <= 1 ? 1 : 0, Ri.p, flag, st);
       Y = mm_cm(cm(Y.p, n, k), rm(Ri.p, k, k));
-      if (pass == 0) add_noise<T>(Y.p, n * k, 1e-14 / std::sqrt(static_cast<double>(n)), ++noise_stream, st);
+      if (pass == 0) add_noise<T>(Y.p, n * k, 1e-14 / std::sqrt(static_cast<double>(n)), ++*keys, st);
     }
   }
 
@@ -950,6 +955,11 @@ struct EngineT final : Engine {
     int64_t nrow, ncol;
     int key, b, w;
     double* host;  // page-locked: b singular values, w residuals, the pivot flag
+    // The row's own, so that its solve does not depend on the others that run
+    // between its steps: the pivot flag, and (keep_order aside, whose rows take no
+    // turns) the count of its perturbations.
+    DT<int> pivot;
+    uint64_t keys;
     // Attempt 0 orthonormalises by shifted CholeskyQR.  A matrix of rank below
     // the block (the padded environments of an iTPO, whose single-layer
     // matrices are narrow) can leave a Gram matrix that no shift makes
@@ -968,16 +978,19 @@ struct EngineT final : Engine {
     ExactSolve(EngineT* e_, const DT<T>& M_, int64_t nrow_, int64_t ncol_, int b_, double* host_)
         : e(e_), M(M_), nrow(nrow_), ncol(ncol_), key(e_->proj_key), b(b_), host(host_) {
       w = static_cast<int>(std::min<int64_t>(e->P.chi, std::min(nrow, ncol)));
+      pivot = DT<int>({1}, e->st);
+      keys = static_cast<uint64_t>(key + 1) << 32;
       ++e->exact_solves;
       start();
     }
     void orth(DT<T>& X, int64_t n, int passes) {
       if (householder) e->orth_cm(X, n, b);
-      else e->orth_chol(X, n, b, passes, !e->keep_order());
+      else e->orth_chol(X, n, b, passes, !e->keep_order(), pivot.p, e->keep_order() ? nullptr : &keys);
     }
     void start() {
       PrecScope fp64(e, 0);
       const MV m = rm(M.p, nrow, ncol);
+      TG_CUDA(cudaMemsetAsync(pivot.p, 0, sizeof(int), e->st));
       DT<T> Om({b, ncol}, e->st);  // column-major ncol x b
       int w0 = 0;
       auto hit = e->warm_v.find(key);
@@ -1021,7 +1034,7 @@ struct EngineT final : Engine {
       ritz_residual<T>(MV1.p, U1.p, s.p, nrow, w, r.p, e->st);
       TG_CUDA(cudaMemcpyAsync(host, s.p, sizeof(double) * b, cudaMemcpyDeviceToHost, e->st));
       TG_CUDA(cudaMemcpyAsync(host + b, r.p, sizeof(double) * w, cudaMemcpyDeviceToHost, e->st));
-      TG_CUDA(cudaMemcpyAsync(host + b + w, e->d_flag + e->slot, sizeof(int), cudaMemcpyDeviceToHost, e->st));
+      TG_CUDA(cudaMemcpyAsync(host + b + w, pivot.p, sizeof(int), cudaMemcpyDeviceToHost, e->st));
     }
     State check() {
       TG_CUDA(cudaStreamSynchronize(e->st));
@@ -1029,7 +1042,6 @@ struct EngineT final : Engine {
       int pivot_flag;
       std::memcpy(&pivot_flag, host + b + w, sizeof(int));
       if (pivot_flag) {  // an orthonormalisation met a non-positive pivot
-        TG_CUDA(cudaMemsetAsync(e->d_flag + e->slot, 0, sizeof(int), e->st));
         if (householder) return failed();
         householder = true;
         start();

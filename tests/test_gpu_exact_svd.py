@@ -3,6 +3,7 @@ subspace iteration."""
 import numpy as np
 import pytest
 
+from tenes_b200 import _lib
 from tenes_b200.env import CTMParams, Environment
 
 pytestmark = pytest.mark.gpu
@@ -64,3 +65,26 @@ def test_from_scratch_whatever_was_before(D, chi, is_complex, density):
         assert counts == got[0][0]
         for a, b in zip(tensors, got[0][1]):
             assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("falloff,is_complex", [(6.0, True), (6.0, False), (0.5, False)])
+def test_rows_do_not_depend_on_each_other(falloff, is_complex):
+    """Six rows whose solves take turns on four streams give what they give one
+    after the other, as they run under the profiler, bit for bit and with the
+    same iterations.  The steep tensors' panels are rank deficient: CholeskyQR
+    meets a pivot that is not positive in some of the rows."""
+    dims = [[3] * 4] * 12
+    tensors = site_tensors(dims, 7, falloff, is_complex)
+    got = []
+    for one_by_one in (0, 1):
+        _lib.load().tg_profile_enable(one_by_one)
+        try:
+            env = Environment(2, 6, [2] * 12, dims,
+                              CTMParams(chi=16, max_ctm_iteration=2, ctm_convergence_epsilon=1e-10), is_complex)
+            got.append((run(env, tensors), [env.get_env(w, i) for w in range(8) for i in range(12)]))
+            env.close()
+        finally:
+            _lib.load().tg_profile_enable(0)
+    assert got[0][0]["solves"] == 96 and got[0][0] == got[1][0]
+    for a, b in zip(got[0][1], got[1][1]):
+        assert np.array_equal(a, b)

@@ -16,10 +16,12 @@ namespace tg {
 //
 // Otherwise the first check is where the projector's last solve in this
 // environment ended, the next ones come from the decay seen between two checks
-// or, before there are two, expected from the block's spectrum.  Against the
-// fixed places, 2 x 2 environments of D = 3 and 4, real and complex, 60 inputs:
-// 0.79 of the time, errors against 64 bits 1.3e-14 to 9.9e-14 against 1.1e-14 to
-// 8.1e-14 (geometric means of 12).
+// or, before there are two, expected from the block's spectrum, with one iteration
+// in hand: without it the first sweeps' solves ended close below the tolerance,
+// and the density matrices of 2 x 2, D = 3 complex environments of chi = 25, 27 and
+// 29 were 1.2e-13, 2.5e-13 and 2.3e-13 off those in 64 bits (geometric means of 8);
+// with it 0.8e-13, 1.6e-13 and 1.3e-13, at fixed places 0.7e-13, 0.8e-13 and 1.9e-13
+// (a second run of a context 2.0e-13, 1.3e-13 and 3.3e-13), in 0.8 of the time.
 struct ExactSteps {
   static constexpr int kMaxIters = 80;
 
@@ -43,7 +45,9 @@ struct ExactSteps {
     const double f = decay(it, ratio, edge);
     const double need = f > 0.0 ? std::max(1.0, std::ceil(std::log(ratio) / -std::log(f))) : 3.0;
     const int left = kMaxIters - it;
-    int gap = falling(ratio) || (prev_it == 0 && !fixed) ? static_cast<int>(std::min(16.0, need)) : 3;
+    int gap = 3;
+    if (falling(ratio)) gap = static_cast<int>(std::min(16.0, need));
+    else if (prev_it == 0 && !fixed) gap = static_cast<int>(std::min(16.0, need + 1.0));
     if (fixed) {
       if (prev_it > 0 && it > 12 && ratio > 0.5 * prev_ratio) return 0;
     } else {

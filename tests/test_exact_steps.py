@@ -46,6 +46,15 @@ def test_ends_where_the_decay_allows(solve):
         assert hint == 2 or 0 <= it - hint <= 2
 
 
+def test_first_gap_has_an_iteration_in_hand(solve):
+    """A solve without a hint that decays as its spectrum promises ends below
+    the tolerance by an iteration's decay (or at its first check)."""
+    cases = [(0, warm, 0, ratio0, decay, decay) for warm in (0, 1) for ratio0 in (1e2, 1e4) for decay in (0.2, 0.45)]
+    for c, (it, checks, ratio, hint) in zip(cases, solve(cases)):
+        assert checks == 1 or ratio <= c[4] * (1 + 1e-12), c
+    assert max(checks for it, checks, ratio, hint in solve(cases)) > 1
+
+
 def test_hints_settle_on_one_check(solve):
     """Solves that hand their hints on need one check each, no more than one
     iteration from the first that ends."""

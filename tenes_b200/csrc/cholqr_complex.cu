@@ -288,7 +288,7 @@ __global__ void __launch_bounds__(ZQ_THREADS, 1)
     cluster.sync();
     // ---- 3. CTA 0: gather, equilibrate, shift, factor
     if (rank == 0) {
-for (int e = tid; e < total; e += ZQ_THREADS) {
+      for (int e = tid; e < total; e += ZQ_THREADS) {
         const int owner = e / per;
         if (owner != 0) {
           const int off = entry(e);

@@ -562,10 +562,9 @@ void launch_w(const Rot<CPLX>* log, const int* info, int n, bool circle, void* W
     ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
     kernel<<<(n + kWRows - 1) / kWRows, 32 * kWRows, smem, st>>>(log, info, n, circle, W);
   };
-  // slots: the groups of a round over the lanes
+  // slots: the groups of a round (at most 60) over the lanes
   if (sch.groups <= 32) go(jacobi_w_kernel<CPLX, 1, 8>);
-  else if (sch.groups <= 64) go(jacobi_w_kernel<CPLX, 2, CPLX ? 4 : 6>);
-  else go(jacobi_w_kernel<CPLX, 3, 4>);
+  else go(jacobi_w_kernel<CPLX, 2, CPLX ? 4 : 6>);
   TG_CHECK_LAUNCH();
   count_launch();
 }
@@ -591,8 +590,9 @@ void launch_jacobi(const void* A, const void* const* mats, int count, int n, voi
   else if (n <= 48) go(jacobi_kernel<CPLX, 16, 3, MODE, 448, false>, 16, 3, 0);
   else if (n <= 64) go(jacobi_kernel<CPLX, 16, 4, MODE, 576, false>, 16, 4, 0);
   else if (n <= kMaxResident) go(jacobi_kernel<CPLX, 16, 6, MODE, 800, false>, 16, 6, 0);
-  else if constexpr (CPLX) go(jacobi_kernel<CPLX, 8, 15, MODE, 256, true>, 8, 15, 256);
-  else go(jacobi_kernel<CPLX, 8, 21, MODE, 512, true>, 8, 21, 512);
+  else if constexpr (!CPLX) go(jacobi_kernel<CPLX, 8, 21, MODE, 512, true>, 8, 21, 512);
+  else if constexpr (MODE == kSpectrum) go(jacobi_kernel<CPLX, 8, 15, MODE, 256, true>, 8, 15, 256);
+  else fail(TG_E_INPUT, "jacobi: n out of range");  // complex SVDs stop at jacobi_svd_max_k
   TG_CHECK_LAUNCH();
   count_launch();
 }

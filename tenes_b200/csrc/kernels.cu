@@ -1546,15 +1546,14 @@ __global__ void upper_to_rh_kernel(const T* __restrict__ acm, int64_t lda, int64
   }
 }
 
-// sum of |x|^2 over a shared-memory array (re [, im] planes), whole CTA
-template <bool CPLX>
+// sum of |x|^2 over a shared-memory array (re, im planes), whole CTA
 __device__ double block_sumsq(const double* re, const double* im, int len) {
   __shared__ double wsum[32];
   __shared__ double total;
   double a = 0.0;
   for (int i = threadIdx.x; i < len; i += blockDim.x) {
     a += re[i] * re[i];
-    if constexpr (CPLX) a += im[i] * im[i];
+    a += im[i] * im[i];
   }
   for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
   if ((threadIdx.x & 31) == 0) wsum[threadIdx.x >> 5] = a;
@@ -1570,49 +1569,47 @@ __device__ double block_sumsq(const double* re, const double* im, int len) {
 
 // One-sided Jacobi SVD with vectors, for the complex matrices of the randomised
 // projectors; see jacobi_svd_complex() in kernels.cuh.
-// Column pairs of a round-robin schedule are handled by groups of kJG lanes;
-// lane gl of a group holds rows gl + kJG i (i < RPL) of the pair's two
+// Column pairs of a round-robin schedule are handled by groups of 16 lanes;
+// lane gl of a group holds rows gl + 16 i (i < RPL) of the pair's two
 // columns in registers for the round: one batch of loads, the dot product,
 // the rotation and the update in registers, one batch of stores (the right
-// vectors are loaded only for pairs that rotate).  Squared column norms are
+// vectors are loaded only for pairs that rotate, in the update: the registers
+// do not hold them earlier).  Squared column norms are
 // exact at the start of every sweep and updated with each rotation
 // (alpha' = alpha - t g, beta' = beta + t g).
-template <typename T, bool CPLX, int kJG, int RPL>
-__global__ void __launch_bounds__(kJG == 16 ? 768 : 1024) jacobi_svd_kernel(const T* __restrict__ A, int n, T* __restrict__ U,
-                                                          double* __restrict__ S, T* __restrict__ Wout,
-                                                          const T* __restrict__ Winit) {
+constexpr int kJG = 16;
+template <int RPL>
+__global__ void __launch_bounds__(768) jacobi_svd_kernel(const cplx* __restrict__ A, int n, cplx* __restrict__ U,
+                                                         double* __restrict__ S, cplx* __restrict__ Wout) {
   extern __shared__ double sm[];
   const int nn = n * n;
   double* ar = sm;
-  double* ai = sm + nn;                       // complex only
-  double* wr = sm + (CPLX ? 2 : 1) * nn;
-  double* wi = wr + nn;                       // complex only
-  double* nrm = sm + (CPLX ? 4 : 2) * nn;     // n
+  double* ai = ar + nn;
+  double* wr = ai + nn;
+  double* wi = wr + nn;
+  double* nrm = wi + nn;                       // n
   int* pos = reinterpret_cast<int*>(nrm + n);  // n
   __shared__ int rotated;
   for (int idx = threadIdx.x; idx < nn; idx += blockDim.x) {
     const int r = idx / n, c = idx % n;
-    const T v = A[idx];
-    ar[c * n + r] = re_of(v);
-    const T w0 = Winit ? Winit[idx] : ((r == c) ? one_of<T>() : zero_of<T>());
-    wr[c * n + r] = re_of(w0);
-    if constexpr (CPLX) {
-      ai[c * n + r] = im_of(v);
-      wi[c * n + r] = im_of(w0);
-    }
+    const cplx v = A[idx];
+    ar[c * n + r] = v.x;
+    ai[c * n + r] = v.y;
+    wr[c * n + r] = r == c ? 1.0 : 0.0;
+    wi[c * n + r] = 0.0;
   }
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int np = n + (n & 1);
   const double tol = static_cast<double>(n) * 2.220446049250313e-16, tol2 = tol * tol;
-  const double small2 = tol * tol * block_sumsq<CPLX>(ar, ai, nn);  // rounding-noise columns
+  const double small2 = tol * tol * block_sumsq(ar, ai, nn);  // rounding-noise columns
   const int grp = lane / kJG, gl = lane % kJG;
   for (int sweep = 0; sweep < 60; ++sweep) {
     for (int c = warp; c < n; c += nw) {
       double a = 0;
       for (int r = lane; r < n; r += 32) {
         a += ar[c * n + r] * ar[c * n + r];
-        if constexpr (CPLX) a += ai[c * n + r] * ai[c * n + r];
+        a += ai[c * n + r] * ai[c * n + r];
       }
       for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
       if (lane == 0) nrm[c] = a;
@@ -1640,88 +1637,63 @@ __global__ void __launch_bounds__(kJG == 16 ? 768 : 1024) jacobi_svd_kernel(cons
             q = t;
           }
         }
-        double xp[RPL], xq[RPL], yp[CPLX ? RPL : 1], yq[CPLX ? RPL : 1];
+        double xp[RPL], xq[RPL], yp[RPL], yq[RPL];
 #pragma unroll
         for (int i = 0; i < RPL; ++i) {
           const int r = gl + i * kJG;
           const bool ok = valid && r < n;
           xp[i] = ok ? ar[p * n + r] : 0.0;
           xq[i] = ok ? ar[q * n + r] : 0.0;
-          if constexpr (CPLX) {
-            yp[i] = ok ? ai[p * n + r] : 0.0;
-            yq[i] = ok ? ai[q * n + r] : 0.0;
-          }
+          yp[i] = ok ? ai[p * n + r] : 0.0;
+          yq[i] = ok ? ai[q * n + r] : 0.0;
         }
         double gr = 0, gi = 0, gr2 = 0, gi2 = 0;  // two accumulators: shorter FP64 chains
 #pragma unroll
         for (int i = 0; i < RPL; ++i) {
           double& a = (i & 1) ? gr2 : gr;
+          double& b = (i & 1) ? gi2 : gi;
           a = fma(xp[i], xq[i], a);
-          if constexpr (CPLX) {
-            double& b = (i & 1) ? gi2 : gi;
-            a = fma(yp[i], yq[i], a);
-            b = fma(xp[i], yq[i], b);
-            b = fma(-yp[i], xq[i], b);
-          }
+          a = fma(yp[i], yq[i], a);
+          b = fma(xp[i], yq[i], b);
+          b = fma(-yp[i], xq[i], b);
         }
         gr += gr2;
         gi += gi2;
 #pragma unroll
         for (int o = kJG / 2; o > 0; o >>= 1) {  // reduce within the lane group
           gr += __shfl_xor_sync(0xffffffffu, gr, o, kJG);
-          if constexpr (CPLX) gi += __shfl_xor_sync(0xffffffffu, gi, o, kJG);
+          gi += __shfl_xor_sync(0xffffffffu, gi, o, kJG);
         }
         const double al = valid ? nrm[p] : 0.0, be = valid ? nrm[q] : 0.0;
-        const double g = CPLX ? hypot(gr, gi) : fabs(gr);
+        const double g = hypot(gr, gi);
         if (!valid || g == 0.0 || al <= small2 || be <= small2 || g * g <= tol2 * al * be) continue;
-        // real: the right vectors of the pair, issued before the rotation
-        // arithmetic; complex: loaded in the update (register budget)
-        double vp[CPLX ? 1 : RPL], vq[CPLX ? 1 : RPL];
-        if constexpr (!CPLX) {
-#pragma unroll
-          for (int i = 0; i < RPL; ++i) {
-            const int r = gl + i * kJG;
-            const bool ok = r < n;
-            vp[i] = ok ? wr[p * n + r] : 0.0;
-            vq[i] = ok ? wr[q * n + r] : 0.0;
-          }
-        }
         // b = phase * a_q with a_p . b = g > 0; the rotation that zeroes it has
         // t = sign(tau) 2g / (|tau| + sqrt(tau^2 + 4 g^2)), tau = beta - alpha
         // (the smaller root of t^2 + 2 zeta t - 1 = 0, zeta = tau / 2g), in
         // rsqrt steps only; c = 1 / sqrt(1 + t^2) keeps c^2 + s^2 = 1 to
         // rounding whatever the accuracy of t
-        const double ph_r = CPLX ? gr / g : (gr >= 0 ? 1.0 : -1.0);
-        const double ph_i = CPLX ? -gi / g : 0.0;
+        const double ph_r = gr / g, ph_i = -gi / g;
         const double tau = be - al;
         const double w = fma(tau, tau, 4.0 * g * g);
         const double den = fabs(tau) + w * rsqrt(w);
         const double rd = rsqrt(den);
         const double t = copysign(2.0 * g, tau) * (rd * rd);
         const double c = rsqrt(fma(t, t, 1.0)), s = c * t;
-        const double sph = s * ph_r, cph = c * ph_r;
 #pragma unroll
         for (int i = 0; i < RPL; ++i) {
           const int r = gl + i * kJG;
           if (r < n) {
-            if constexpr (CPLX) {
-              const double bqr = xq[i] * ph_r - yq[i] * ph_i, bqi = xq[i] * ph_i + yq[i] * ph_r;
-              ar[p * n + r] = c * xp[i] - s * bqr;
-              ar[q * n + r] = s * xp[i] + c * bqr;
-              ai[p * n + r] = c * yp[i] - s * bqi;
-              ai[q * n + r] = s * yp[i] + c * bqi;
-              const double vpr = wr[p * n + r], vqr = wr[q * n + r], vpi = wi[p * n + r], vqi = wi[q * n + r];
-              const double dqr = vqr * ph_r - vqi * ph_i, dqi = vqr * ph_i + vqi * ph_r;
-              wr[p * n + r] = c * vpr - s * dqr;
-              wr[q * n + r] = s * vpr + c * dqr;
-              wi[p * n + r] = c * vpi - s * dqi;
-              wi[q * n + r] = s * vpi + c * dqi;
-            } else {  // ph_r = +-1 folded into the coefficients (exact)
-              ar[p * n + r] = c * xp[i] - sph * xq[i];
-              ar[q * n + r] = s * xp[i] + cph * xq[i];
-              wr[p * n + r] = c * vp[i] - sph * vq[i];
-              wr[q * n + r] = s * vp[i] + cph * vq[i];
-            }
+            const double bqr = xq[i] * ph_r - yq[i] * ph_i, bqi = xq[i] * ph_i + yq[i] * ph_r;
+            ar[p * n + r] = c * xp[i] - s * bqr;
+            ar[q * n + r] = s * xp[i] + c * bqr;
+            ai[p * n + r] = c * yp[i] - s * bqi;
+            ai[q * n + r] = s * yp[i] + c * bqi;
+            const double vpr = wr[p * n + r], vqr = wr[q * n + r], vpi = wi[p * n + r], vqi = wi[q * n + r];
+            const double dqr = vqr * ph_r - vqi * ph_i, dqi = vqr * ph_i + vqi * ph_r;
+            wr[p * n + r] = c * vpr - s * dqr;
+            wr[q * n + r] = s * vpr + c * dqr;
+            wi[p * n + r] = c * vpi - s * dqi;
+            wi[q * n + r] = s * vpi + c * dqi;
           }
         }
         if (gl == 0) {
@@ -1740,7 +1712,7 @@ __global__ void __launch_bounds__(kJG == 16 ? 768 : 1024) jacobi_svd_kernel(cons
     double a = 0;
     for (int r = lane; r < n; r += 32) {
       a += ar[c * n + r] * ar[c * n + r];
-      if constexpr (CPLX) a += ai[c * n + r] * ai[c * n + r];
+      a += ai[c * n + r] * ai[c * n + r];
     }
     for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
     if (lane == 0) nrm[c] = sqrt(a);
@@ -1761,13 +1733,8 @@ __global__ void __launch_bounds__(kJG == 16 ? 768 : 1024) jacobi_svd_kernel(cons
     const int r = idx / n, c = idx % n;  // source column c -> output column pos[c]
     const double inv = nrm[c] > 0.0 ? 1.0 / nrm[c] : 0.0;
     const int64_t o = static_cast<int64_t>(r) * n + pos[c];
-    if constexpr (CPLX) {
-      U[o] = make_double2(ar[c * n + r] * inv, ai[c * n + r] * inv);
-      Wout[o] = make_double2(wr[c * n + r], wi[c * n + r]);
-    } else {
-      U[o] = ar[c * n + r] * inv;
-      Wout[o] = wr[c * n + r];
-    }
+    U[o] = make_double2(ar[c * n + r] * inv, ai[c * n + r] * inv);
+    Wout[o] = make_double2(wr[c * n + r], wi[c * n + r]);
   }
 }
 
@@ -2875,14 +2842,14 @@ void jacobi_svd_complex(const cplx* A, int64_t k, cplx* U, double* S, cplx* W, c
   const int npairs = static_cast<int>((k + 1) / 2);
   auto run = [&](auto kernel) {
     ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
-    const int threads = static_cast<int>(std::min<int64_t>(1024, (static_cast<int64_t>(npairs) * 16 + 31) / 32 * 32));
-    kernel<<<1, threads, smem, st>>>(A, static_cast<int>(k), U, S, W, nullptr);
+    const int threads = static_cast<int>(std::min<int64_t>(1024, (static_cast<int64_t>(npairs) * kJG + 31) / 32 * 32));
+    kernel<<<1, threads, smem, st>>>(A, static_cast<int>(k), U, S, W);
   };
   // rows a lane holds: the fewest that cover k (masked rows add exact zeros,
   // so the sums -- and the result -- are those of any larger choice)
-  if (k <= 48) run(jacobi_svd_kernel<cplx, true, 16, 3>);
-  else if (k <= 64) run(jacobi_svd_kernel<cplx, true, 16, 4>);
-  else run(jacobi_svd_kernel<cplx, true, 16, 6>);
+  if (k <= 48) run(jacobi_svd_kernel<3>);
+  else if (k <= 64) run(jacobi_svd_kernel<4>);
+  else run(jacobi_svd_kernel<6>);
   TG_CHECK_LAUNCH();
   count_launch();
 }

@@ -72,9 +72,10 @@ typedef struct tg_params {
                                        3xTF32 tensor-core products (FP64 tile accumulation); the
                                        orthonormalisation, SVDs and observables stay FP64.  Real
                                        tensors only.  0 (default): everything FP64. */
-  int cuda_graph;                   /* 1 (default): with rSVD corner projectors, replay each CTMRG
-                                       sweep from a captured CUDA graph (same kernels, same results);
-                                       0: launch every kernel from the host. */
+  int cuda_graph;                   /* 1 (default): where no projector waits for the host (randomised
+                                       ones, small full-SVD ones), replay each CTMRG sweep from a
+                                       captured CUDA graph (same kernels, same results); 0: launch
+                                       every kernel from the host. */
   int svd_solver;                   /* solver of the full-SVD projectors (use_rsvd = 0,
                                        ctm.cpp:267-302, 441-475): 0 (default) the leading singular
                                        triplets the truncation keeps, by block subspace iteration
@@ -161,6 +162,10 @@ tg_status tg_ctm_check_convergence(tg_ctx* ctx, int* converged, double* sig_max)
  * out[2] Rayleigh-Ritz checks, out[3] solves handed to the dense SVD.
  * Cumulative over the context's life. */
 tg_status tg_projector_svd_stats(tg_ctx* ctx, int64_t* out);
+
+/* Counters of the sweeps' CUDA graph (tg_params.cuda_graph): out[0] sweeps
+ * replayed, out[1] captures.  Cumulative over the context's life. */
+tg_status tg_ctm_graph_stats(tg_ctx* ctx, int64_t* out);
 
 /* core::Calc_CTM_Environment (ctm.cpp:971-1253): optional init, then sweeps
  * until converged or max_ctm_iteration.  Returns TG_OK also when not

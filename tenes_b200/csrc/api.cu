@@ -158,6 +158,12 @@ tg_status tg_projector_svd_stats(tg_ctx* ctx, int64_t* out) {
     E(ctx)->svd_stats(out);
   });
 }
+tg_status tg_ctm_graph_stats(tg_ctx* ctx, int64_t* out) {
+  return guard([&] {
+    need(out, "out");
+    E(ctx)->graph_stats(out);
+  });
+}
 tg_status tg_ctm_run(tg_ctx* ctx, int initialize, int* iterations, int* converged, double* sig_max) {
   return guard([&] { E(ctx)->ctm_run(initialize, iterations, converged, sig_max); });
 }

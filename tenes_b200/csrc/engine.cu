@@ -1819,7 +1819,8 @@ struct EngineT final : Engine {
   std::vector<const void*> g_addr;
   uint64_t g_kernels = 0;
   int g_infos = 0;  // cuSOLVER status slots that a replay writes
-  int g_eager = 0;  // sweeps run eagerly since the last change
+  int g_eager = 0;  // sweeps run eagerly since the context began or a graph was dropped
+  int64_t graph_replays = 0, graph_captures = 0;
   bool g_broken = false;
 
   std::vector<const void*> state_addresses() {
@@ -1914,6 +1915,7 @@ struct EngineT final : Engine {
       return;
     }
     g_addr = state_addresses();
+    ++graph_captures;
   }
 
   // `left`: sweeps that may still come, this one included
@@ -1938,6 +1940,7 @@ struct EngineT final : Engine {
     }
     if (g_infos > 0) check_infos();  // the slots the replay is about to write
     TG_CUDA(cudaGraphLaunch(g_exec, st));
+    ++graph_replays;
     info_used = g_infos;
     count_launch(g_kernels);
   }
@@ -3389,6 +3392,10 @@ struct EngineT final : Engine {
     out[1] = exact_iters;
     out[2] = exact_checks;
     out[3] = exact_dense;
+  }
+  void graph_stats(int64_t* out) override {
+    out[0] = graph_replays;
+    out[1] = graph_captures;
   }
 
   void sync() override {

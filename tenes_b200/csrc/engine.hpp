@@ -48,6 +48,7 @@ struct Engine {
   // counters of the exact truncated SVD of the full-SVD projectors:
   // solves, subspace iterations, Rayleigh-Ritz checks, dense fallbacks
   virtual void svd_stats(int64_t* out) = 0;
+  virtual void graph_stats(int64_t* out) = 0;
   virtual void sync() = 0;
   virtual void* stream() = 0;
 };

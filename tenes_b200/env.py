@@ -186,6 +186,12 @@ class Environment:
         check(self.lib.tg_projector_svd_stats(self.ctx, out))
         return {"solves": out[0], "iterations": out[1], "checks": out[2], "dense": out[3]}
 
+    def graph_stats(self) -> dict:
+        """Counters of the sweeps' CUDA graph."""
+        out = (C.c_int64 * 2)()
+        check(self.lib.tg_ctm_graph_stats(self.ctx, out))
+        return {"replays": out[0], "captures": out[1]}
+
     def corner_spectrum(self, which: int, i: int) -> np.ndarray:
         a = np.empty(self.params.chi, dtype=np.float64)
         check(self.lib.tg_corner_spectrum(self.ctx, which, i, dptr(a)))

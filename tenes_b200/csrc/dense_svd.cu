@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(kQrThreads)
   double* nrm = reinterpret_cast<double*>(a + static_cast<size_t>(ld) * k);
   int* at = reinterpret_cast<int*>(nrm + k);                 // place c holds column at[c]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
-  __shared__ int warp_top[kQrThreads / 32];
+  int* warp_top = reinterpret_cast<int*>(nrm);  // (static shared memory would not fit beside the largest matrices)
   int top = 0;
   for (int idx = tid; idx < m * k; idx += blockDim.x) {
     const int r = sc == 1 ? idx / k : idx % m, c = sc == 1 ? idx % k : idx / m;
@@ -87,11 +87,10 @@ __global__ void __launch_bounds__(kQrThreads)
   top = __reduce_max_sync(0xffffffffu, lane < nw ? warp_top[lane] : 0);
   double unscale;
   const double range = range_scale(top, unscale);
-  if (range != 1.0) {  // the same in every thread
+  if (range != 1.0)  // the same in every thread
     for (int idx = tid; idx < ld * k; idx += blockDim.x)
       if (idx % ld < m) a[idx] = times(a[idx], range);
-    __syncthreads();
-  }
+  __syncthreads();  // also before warp_top's place takes the norms
   if (tid == 0 && top >= 0x7ff00000 && info) atomicExch(info, 1);
   for (int c = warp; c < k; c += nw) {
     double s = 0.0;
@@ -240,7 +239,9 @@ __global__ void __launch_bounds__(128)
 
 template <typename T>
 size_t qr_smem(int64_t m, int64_t k) {
-  return sizeof(T) * static_cast<size_t>((m | 1) * k) + (sizeof(double) + sizeof(int)) * static_cast<size_t>(k);
+  // the norms' place also holds a value of every warp
+  return sizeof(T) * static_cast<size_t>((m | 1) * k) +
+         std::max((sizeof(double) + sizeof(int)) * static_cast<size_t>(k), sizeof(int) * (kQrThreads / 32));
 }
 
 }  // namespace

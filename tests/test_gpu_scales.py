@@ -55,7 +55,7 @@ def dense_svd(A):
 
 
 @pytest.mark.parametrize("is_complex", [False, True])
-@pytest.mark.parametrize("m,n", [(12, 12), (33, 20), (40, 90)])
+@pytest.mark.parametrize("m,n", [(1, 1), (12, 12), (33, 20), (40, 90), (201, 72)])  # 201 x 72 complex: all but 32 B of 227 KB
 def test_dense_svd(m, n, is_complex):
     A = matrix(max(m, n), is_complex, m + n)[:m, :n]
     tol = 40 * min(m, n) * U * np.linalg.norm(A)  # the bound at unit scale (test_gpu_dense_svd.py)

@@ -30,10 +30,7 @@ struct ExactSteps {
   double prev_ratio = 0.0;
 
   // the first check; hint: hint() of the projector's last solve, 0: none
-  int first(bool warm, int hint) const {
-    if (fixed) return warm ? 1 : 3;
-    return hint > 0 ? hint : warm ? 2 : 3;
-  }
+  int first(bool warm, int hint) const { return !fixed && hint > 0 ? hint : warm ? 1 : 3; }
   bool falling(double ratio) const { return prev_it > 0 && ratio < prev_ratio; }
   // the residuals' decay an iteration; edge: the same expected from the spectrum
   double decay(int it, double ratio, double edge) const {
@@ -70,7 +67,7 @@ struct ExactSteps {
     const double f = decay(it, ratio, edge);
     int spare = 0;
     while (spare < 2 && f > 0.0 && ratio * std::pow(f, -(spare + 1)) <= 1.0) ++spare;
-    return std::max(2, it - spare);
+    return std::max(1, it - spare);
   }
 };
 

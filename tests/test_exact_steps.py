@@ -43,7 +43,7 @@ def test_ends_where_the_decay_allows(solve):
         need = math.log(c[3]) / -math.log(c[4])
         assert it > 0 and ratio <= 1.0, c
         assert it <= max(c[2], 3, need) + 16, c
-        assert hint == 2 or 0 <= it - hint <= 2
+        assert hint >= 1 and 0 <= it - hint <= 2
 
 
 def test_first_gap_has_an_iteration_in_hand(solve):
@@ -63,7 +63,17 @@ def test_hints_settle_on_one_check(solve):
         for _ in range(30):
             it, checks, ratio, hint = solve([(0, 1, hint, ratio0, decay, decay)])[0]
         need = math.ceil(math.log(ratio0) / -math.log(decay))
-        assert checks == 1 and it - need <= 1 or it == 2, (ratio0, decay, it)
+        assert checks == 1 and it - need <= 1, (ratio0, decay, it)
+
+
+def test_hints_reach_one(solve):
+    """Where one iteration is enough, the next solves look there."""
+    for ratio0, decay in ((1e-3, 0.5), (0.5, 0.1), (5.0, 0.1)):
+        hint = 7
+        for _ in range(10):
+            it, checks, ratio, hint = solve([(0, 1, hint, ratio0, decay, decay)])[0]
+        assert (it, checks) == (1, 1)
+    assert solve([(0, 1, 0, 0.5, 0.1, 0.1)])[0][:2] == (1, 1)
 
 
 def test_flat_spectra_are_given_up(solve):

@@ -571,10 +571,12 @@ void launch_w(const Rot<CPLX>* log, const int* info, int n, bool circle, void* W
 
 // LANES x RPL covers the rows; 16 lanes a column and a group a pair up to 96
 // columns (with 8 lanes and 16-byte accesses 48 columns took 145 us against
-// 135, 96 columns 556 against 541).  Above, 8 lanes hold a column without
-// spilling in 512 (complex 256) threads, which take the pairs of a round in two
-// or three turns: 162 columns took 18.8 ms spilling with a whole round at once,
-// 6.5 ms so.
+// 135, 96 columns 556 against 541).  Above, 8 lanes hold a column in 512
+// (complex 256) threads, which take the pairs of a round in two or three turns:
+// the one form that reaches the 160 columns of a spectrum without spilling.  119
+// columns take 2.52 ms so (and spectra of 109 columns 2.42 ms, against 7.29 ms a
+// warp a pair); a whole round at once on 16 lanes of 8 rows, up to 119 columns,
+// was measured at 1.42 and 1.15 ms and is not built.
 constexpr int kMaxResident = 96;
 template <bool CPLX, int MODE>
 void launch_jacobi(const void* A, const void* const* mats, int count, int n, void* U, double* S, Rot<CPLX>* log,

@@ -902,10 +902,11 @@ struct EngineT final : Engine {
   // The start block holds the basis that the same projector (move, line,
   // row) ended with in the previous sweep -- an almost converged guess once
   // the environment settles -- completed with counter-based Gaussian
-  // columns.  An environment made from the site tensors, or set, starts without
-  // them (forget_solves), so that it does not depend on what the context computed
+  // columns.  An environment made from the site tensors starts without them
+  // (forget_solves), so that it does not depend on what the context computed
   // before; only keep_order() contexts keep them, as their results would move
-  // with the start block.  If the residuals are not below the tolerance after
+  // with the start block.  (tg_set_env keeps them: a host that holds the
+  // environment itself sets it before every sweep.)  If the residuals are not below the tolerance after
   // ExactSteps::kMaxIters iterations (a flat spectrum at the block edge), the
   // dense SVD is used instead.
   // Contexts whose results carry the last bits of a singular vector to more
@@ -3384,7 +3385,6 @@ struct EngineT final : Engine {
   }
   void set_env(int which, int site, const double* host) override {
     upload(env_ref(which, site), host);  // into the existing storage (captured sweeps hold its address)
-    forget_solves();
     env_ready = true;
     spec_old_ok = false;
   }
